@@ -189,7 +189,7 @@ int fv2d_create(const fv2d_mesh_desc* desc, const fv2d_case* cs, int precision, 
     h->precision = precision;
     h->s.reset(precision == FV2D_FP64 ? fv2d::make_solver_fp64() : fv2d::make_solver_fp32());
     std::string err;
-    rc = fv2d::build_mesh(desc, cs, h->s->mesh_, err);
+    rc = fv2d::build_mesh(desc, cs, h->s->mesh_, err, h->s->side_block(desc ? desc->num_cells : 0));
     if (rc) return fail(rc, err);
     rc = h->s->init(*cs);
     if (rc) return fail(rc, h->s->err_);

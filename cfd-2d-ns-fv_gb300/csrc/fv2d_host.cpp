@@ -343,7 +343,7 @@ void geometry(HostMesh& m) {
     }
 }
 
-void renumber(HostMesh& m) {
+void renumber(HostMesh& m, int block) {
     const int nc = m.nc, nf = m.nf;
     double x0 = m.ccx[0], x1 = m.ccx[0], y0 = m.ccy[0], y1 = m.ccy[0];
     for (int c = 0; c < nc; c++) {
@@ -369,13 +369,12 @@ void renumber(HostMesh& m) {
         key[c] = (d << 32) | (uint32_t)c;
     }
     std::sort(key.begin(), key.end());
-    // Within each run of kSideBlock Hilbert-consecutive cells (a small spatial patch), cells are
+    // Within each run of `block` Hilbert-consecutive cells (a small spatial patch), cells are
     // ordered by face count (stable): a warp's cells then loop over the same number of faces, so
     // the per-cell gathers do not wait for the warp's one many-sided cell.  Results do not depend
     // on the order (every per-cell sum runs in ascending original face id).
-    constexpr int kSideBlock = 256;
-    for (int b0 = 0; b0 < nc; b0 += kSideBlock) {
-        const int b1 = std::min(nc, b0 + kSideBlock);
+    for (int b0 = 0; b0 < nc; b0 += block) {
+        const int b1 = std::min(nc, b0 + block);
         std::stable_sort(key.begin() + b0, key.begin() + b1, [&](uint64_t a, uint64_t b) {
             const int ca = (int)(a & 0xFFFFFFFFu), cb = (int)(b & 0xFFFFFFFFu);
             return m.cf_off[ca + 1] - m.cf_off[ca] < m.cf_off[cb + 1] - m.cf_off[cb];
@@ -405,7 +404,7 @@ void renumber(HostMesh& m) {
 
 }  // namespace
 
-int build_mesh(const fv2d_mesh_desc* d, const fv2d_case* cs, HostMesh& m, std::string& err) {
+int build_mesh(const fv2d_mesh_desc* d, const fv2d_case* cs, HostMesh& m, std::string& err, int block) {
     if (!d || !cs || !d->x || !d->y || !d->face_point1 || !d->face_point2 || !d->face_cell1 || !d->face_cell2) {
         err = "null mesh array"; return FV2D_ERR_ARG;
     }
@@ -426,7 +425,7 @@ int build_mesh(const fv2d_mesh_desc* d, const fv2d_case* cs, HostMesh& m, std::s
             return FV2D_ERR_MESH;
         }
     geometry(m);
-    renumber(m);
+    renumber(m, block);
     return FV2D_OK;
 }
 

@@ -16,6 +16,8 @@ extern const char* const kKernelNames[K_COUNT];
 class Solver {
 public:
     virtual ~Solver() {}
+    // cells per block of the renumbering this engine wants for a mesh of `cells` cells (build_mesh)
+    virtual int side_block(long long cells) { (void)cells; return kSideBlock; }
     virtual int init(const fv2d_case& cs) = 0;       // mesh_ must be set before
     virtual int stage() = 0;
     virtual int step(int iterations) = 0;

@@ -36,22 +36,25 @@ struct TiledImage {
     std::vector<int> n2o;
     long long nc = 0, nc4 = 0, recw = 0, nrec = 0, ncsr = 0, nhalo = 0;
     double rec_per_face = 0, ring1 = 0, ring2 = 0;
+    int max_rec = 0, max_csr = 0, max_halo = 0, max_cells = 0, max_grad = 0, max_flux = 0;   // largest tile
     char* pin = nullptr;
     size_t o_rec = 0, o_qc = 0, o_csr = 0, o_halo = 0, o_vol = 0, o_rvol = 0, o_lsq = 0;
     ~TiledImage() { if (pin) cudaFreeHost(pin); }
 };
 
-int tiled_image(const HostMesh& hm, std::shared_ptr<TiledImage>& out, std::string& err) {
+int tiled_image(const HostMesh& hm, std::shared_ptr<TiledImage>& out, std::string& err, int core = kTileCore) {
     auto& slot = hm.batch_image[1];
     if (slot) { out = std::static_pointer_cast<TiledImage>(slot); return FV2D_OK; }
     DeviceLayout D;
     build_layout(hm, D);
     TileLayout L;
-    if (!build_tile_layout(hm, D, L, err)) return FV2D_ERR_MESH;
+    if (!build_tile_layout(hm, D, L, err, core)) return FV2D_ERR_MESH;
     auto im = std::make_shared<TiledImage>();
     im->nc = L.nc; im->nc4 = L.nc4; im->recw = (long long)L.rec.size(); im->nrec = (long long)L.qcell.size();
     im->ncsr = (long long)L.csr.size(); im->nhalo = (long long)L.halo.size();
     im->rec_per_face = L.rec_per_face; im->ring1 = L.ring1_per_cell; im->ring2 = L.ring2_per_cell;
+    im->max_rec = L.max_rec; im->max_csr = L.max_csr; im->max_halo = L.max_halo;
+    im->max_cells = L.max_cells; im->max_grad = L.max_grad; im->max_flux = L.max_flux;
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
     im->o_rec = take(4 * L.rec.size()); im->o_qc = take(4 * L.qcell.size()); im->o_csr = take(2 * L.csr.size());
@@ -71,6 +74,27 @@ int tiled_image(const HostMesh& hm, std::shared_ptr<TiledImage>& out, std::strin
 }
 
 }  // namespace
+
+// Cells per tile of a single solve (a batch's tiles have kTileCore).  Results do not depend on it.
+// Up to two tiles per SM (77,824 cells on 152 SMs) or three of at most 200 cells (91,200, the most
+// that three CTAs' shared memory holds), the solve runs in the whole-iteration kernel, and the
+// smallest tile that still gives every tile a place is the fastest: its passes are a few dependent
+// loads and divisions long whatever the tile's size, so more tiles means fewer rounds per pass.
+// Below 64 cells the ring cells outweigh that.  Measured, us per iteration: 8,192 quads, tiles of
+// 64 / 128 / 256 cells 12.2 / 13.6 / 18.2 (a stage kernel per stage: 35.4); 50k polygons, 180 / 224
+// / 256: 22.1 / 23.9 / 25.8 (43.5); 88k, 196 (three per SM): 31.7 (44.8).
+// Beyond that the stage kernels take the tiles in waves of three per SM; with only two waves the
+// second is filled by cutting the tiles evenly (120k polygons: 256 -> 136 cells 75.7 -> 66.7 us;
+// 180k: 256 -> 200 76.4 -> 71.6).  From three waves on smaller tiles cost as much in ring cells as the
+// fuller last wave gains (300k: 116.4 -> 116.2; 1M quads 252 -> 258 at 248 cells).
+int solve_tile_cells(long long n, int sms) {
+    auto even = [&](long long tiles) { return (int)round_up((n + tiles - 1) / tiles, 4); };
+    const int t2 = even(2LL * sms), t3 = even(3LL * sms);
+    if (t2 <= kTileCore) return std::max(64, t2);
+    if (t3 <= 200) return t3;
+    const int t6 = even(6LL * sms);
+    return t3 > kTileCore && t6 <= kTileCore ? t6 : kTileCore;
+}
 
 // Arena capacities of the core.
 struct TiledCaps {
@@ -169,6 +193,7 @@ public:
         res2_ = (double*)(a + ores); srange_ = (int*)(a + osr);
         int* misc = (int*)(a + omisc);
         A_.ntiles = misc; A_.counter = misc + 4; A_.err = misc + 8;
+        iter_.bar = (unsigned*)(misc + 32);   // on a cache line of its own
         A_.store_r = 0;
         A_.nsmax = c.solves;
         FV2D_T(cudaMemsetAsync(arena_, 0, bytes_, stream_));
@@ -185,6 +210,63 @@ public:
         int per = 0;
         FV2D_T(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tstage<1>, kTileCore, kSmTotal));
         grid_ = std::max(1, per) * sms_;
+        return FV2D_OK;
+    }
+
+    // The whole-iteration kernel's shared-memory plan for the active solves' largest tiles, and
+    // whether all their tiles fit on the GPU at once.
+    int plan_iter() {
+        TIter p = iter_;
+        p.max_rec = p.max_csr = p.max_halo = p.max_cells = p.max_grad = p.max_flux = 0;
+        for (const Solve& s : solves_) {
+            if (!s.active) continue;
+            const TiledImage& im = *s.image;
+            p.max_rec = std::max(p.max_rec, im.max_rec); p.max_csr = std::max(p.max_csr, im.max_csr);
+            p.max_halo = std::max(p.max_halo, im.max_halo); p.max_cells = std::max(p.max_cells, im.max_cells);
+            p.max_grad = std::max(p.max_grad, im.max_grad); p.max_flux = std::max(p.max_flux, im.max_flux);
+        }
+        int off = 0;
+        auto take = [&](int bytes) { const int o = off; off += (bytes + 15) & ~15; return o; };
+        take(4 * p.max_rec);
+        p.o_csr = take(2 * p.max_csr); p.o_halo = take(4 * p.max_halo); p.o_cq = take(16 * p.max_cells);
+        p.o_cg = take(32 * p.max_grad); p.o_t = take(16 * p.max_flux); p.o_sp = take(4 * p.max_flux);
+        p.o_qp = take(16 * p.max_grad); p.o_lsq = take(16 * p.max_grad);
+        iter_ = p;
+        iter_smem_ = off;
+        iter_planned_ = true;
+        iter_fn_ = nullptr;
+        if (hi_tiles_ <= 0) return FV2D_OK;
+        // two CTAs per SM (no spills) where that holds every tile, else three
+        for (const void* f : {(const void*)k_titer<2>, (const void*)k_titer<3>}) {
+            int per = 0;
+            if (off > kSmTotalMax) continue;
+            FV2D_T(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, off));
+            FV2D_T(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kTileCore, off));
+            if (hi_tiles_ <= (long long)per * sms_) { iter_fn_ = f; break; }
+        }
+        return FV2D_OK;
+    }
+
+    // Up to n iterations by the whole-iteration kernel, in launches of bounded length (other work on
+    // the GPU gets its turn every few milliseconds); *done: those launched, fewer than n only where
+    // such a grid cannot be resident at once (SMs withheld from the process).
+    int launch_iter(int n, int* done) {
+        *done = 0;
+        while (*done < n) {
+            TIter p = iter_;
+            p.iterations = std::min(n - *done, 256);
+            void* args[] = {&A_, &p};
+            const cudaError_t e = cudaLaunchCooperativeKernel(iter_fn_, dim3((unsigned)hi_tiles_), dim3(kTileCore), args,
+                                                              (size_t)iter_smem_, stream_);
+            if (e == cudaErrorCooperativeLaunchTooLarge) {
+                cudaGetLastError();
+                iter_fn_ = nullptr;
+                return FV2D_OK;
+            }
+            FV2D_T(e);
+            iter_.bar0 += (unsigned)hi_tiles_ * (3u * (unsigned)p.iterations - 1u);
+            *done += p.iterations;
+        }
         return FV2D_OK;
     }
 
@@ -340,11 +422,18 @@ public:
         return FV2D_OK;
     }
 
-    // Whole iterations as CUDA-graph replays (captured once; the graphs read the tile list from
+    // Whole iterations: one launch where every tile fits on the GPU at once (k_titer), else as
+    // CUDA-graph replays (captured once; the graphs read the tile list from
     // device memory, so solves join and leave without re-capture): runs of kGraphIters iterations
     // as one replay (fewer gaps between replays), the rest one iteration per replay.
     int iterations(int n, bool graphs) {
         int it = 0;
+        if (n > 0 && graphs && !timing_) {
+            int rc = iter_planned_ ? FV2D_OK : plan_iter();
+            if (!rc && iter_fn_) rc = launch_iter(n, &it);
+            if (rc) return rc;
+            for (auto& s : solves_) if (s.active) s.iterations += it;
+        }
         while (it < n) {
             int k = 1;
             if (!graphs || timing_) {
@@ -384,6 +473,7 @@ public:
         FV2D_T(cudaMemcpy(&e, A_.err, 4, cudaMemcpyDeviceToHost));
         if (e & 2) { err = "a stage kernel's wait for its tile copies timed out"; return FV2D_ERR_CUDA; }
         if (e & 4) { err = "a tile descriptor is out of range"; return FV2D_ERR_CUDA; }
+        if (e & 8) { err = "a barrier between the tiles timed out"; return FV2D_ERR_CUDA; }
         if (flags_out && nflags > 0) FV2D_T(cudaMemcpy(flags_out, A_.flags, 4 * (size_t)nflags, cudaMemcpyDeviceToHost));
         return FV2D_OK;
     }
@@ -467,6 +557,7 @@ private:
         for (int k = 0; k < caps_.solves; k++)
             if (solves_[k].active) hi = std::max<long long>(hi, (long long)solves_[k].first_tile + solves_[k].ntiles);
         *cnt_pin_ = (int)hi;
+        iter_planned_ = false;
         if (full_grid_ && hi != hi_tiles_) drop_graphs();
         hi_tiles_ = hi;
         if (s.ntiles)
@@ -496,6 +587,10 @@ private:
     }
     struct Pending { int kid; cudaEvent_t a, b; };
 
+    TIter iter_{};                       // the whole-iteration kernel's plan for the active solves
+    const void* iter_fn_ = nullptr;      // its variant, null: the tiles do not all fit at once
+    int iter_smem_ = 0;
+    bool iter_planned_ = false;
     void* arena_ = nullptr;
     int* srange_ = nullptr;
     bool keep_r_ = false, norms_ = false, timing_ = false;
@@ -546,12 +641,22 @@ public:
         if (dstage_) cudaFree(dstage_);
     }
 
+    int side_block(long long cells) override {
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
+            cudaGetLastError();
+            return kSideBlock;
+        }
+        return solve_tile_cells(cells, sms);
+    }
+
     int init(const fv2d_case& cs) override {
         cs_ = cs;
         nc_ = mesh_.nc;
         order2_ = cs.order == 2;
         std::shared_ptr<TiledImage> im;
-        int rc = tiled_image(mesh_, im, err_);
+        int rc = tiled_image(mesh_, im, err_, side_block(nc_));   // the tiles are the renumbering's blocks
         if (rc) return rc;
         TiledCaps c;
         c.cells = im->nc4; c.recw = im->recw; c.recs = im->nrec; c.csr = im->ncsr; c.halo = std::max<long long>(4, im->nhalo);

@@ -18,6 +18,8 @@
 // A face shared by two tiles is evaluated by both, with the same inputs and the same code, so both
 // get the same value; every per-cell sum runs in a fixed order, so results do not depend on the
 // tile schedule, and a solve gives the same bits alone and in a batch (both run these kernels).
+// Solves whose tiles all fit on the GPU at once run whole iterations in one launch (k_titer, the same
+// passes).
 #pragma once
 
 #include <cstdint>
@@ -69,6 +71,7 @@ constexpr int kSmHalo = 4 * kTileCells;
 constexpr int kSmCq = 16 * kTileCells;
 constexpr int kSmCg = 32 * kTileGrad;
 constexpr int kSmTotal = kSmRec + kSmCsr + kSmHalo + kSmCq + kSmCg;
+constexpr int kSmTotalMax = 226 * 1024;   // a CTA's limit (227 KB) less its static shared memory
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -117,14 +120,359 @@ __device__ __forceinline__ void copy_async(T* dst, const T* src) {
 }
 
 
+// Every operation of the passes below rounds as written here, so the kernels that share them get the
+// same bits: a product is either rounded by itself (fm, which the compiler does not contract) or
+// the exact operand of a fused multiply-add (ff).
+__device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float fa(float a, float b) { return a + b; }
+__device__ __forceinline__ float fs(float a, float b) { return a - b; }
+__device__ __forceinline__ float ff(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// a*b + c*d with the first product exact
+__device__ __forceinline__ float mm(float a, float b, float c, float d) { return ff(a, b, fm(c, d)); }
+
 // Primitives of a conservative state; returns 1/rho for later quotients.
 __device__ __forceinline__ void tprims(const float p[4], const Consts<float>& k, float& rho, float& u, float& v,
                                        float& P, float& y) {
     rho = p[0];
     y = 1.0f / rho;
-    u = p[1] * y;
-    v = p[2] * y;
-    P = (p[3] - 0.5f * rho * (u * u + v * v)) * k.gm1;
+    u = fm(p[1], y);
+    v = fm(p[2], y);
+    P = fm(ff(-fm(0.5f, rho), mm(u, u, v, v), p[3]), k.gm1);
+}
+// Conservative state of primitives.
+__device__ __forceinline__ void tcons(float rho, float u, float v, float P, const Consts<float>& k, float q[4]) {
+    q[0] = rho;
+    q[1] = fm(rho, u);
+    q[2] = fm(rho, v);
+    q[3] = ff(fm(0.5f, rho), mm(u, u, v, v), P / k.gm1);
+}
+// The no-slip wall's ghost of state p (primitives rho, u, v): velocity negated, the energy rebuilt
+// from the pressure with the kinetic energy's rounded value in both steps.
+__device__ __forceinline__ void tghost_noslip(const float p[4], const Consts<float>& k, float q[4]) {
+    const float rho = p[0], y = 1.0f / rho, u = fm(p[1], y), v = fm(p[2], y);
+    const float ke = mm(u, u, v, v), h = fm(0.5f, rho), m = fm(h, ke);
+    q[0] = rho;
+    q[1] = fm(rho, -u);
+    q[2] = fm(rho, -v);
+    q[3] = ff(fm(fs(p[3], m), k.gm1), 1.0f / k.gm1, m);
+}
+
+// A tile's blocks in shared memory, as the passes read them.
+struct TileView {
+    const uint32_t* sl;               // records: the two cells' local slots
+    const float4* d;                  // records: (d1x, d1y, d2x, d2y)
+    const float *nx, *ny, *A;         // records [0, ngeo)
+    const uint16_t* off;              // csr offsets (bit 15 of an end offset: the cell has a boundary face)
+    const uint32_t* ent;              // csr entries
+    const Q4<float>* cq;              // cell states
+    const Q4<float>* cg;              // limited gradients, (x, y) per core and ring-1 cell
+};
+
+// The limited LSQ gradient of one core or ring-1 cell (local slot gI).  ghost(r): the state of the
+// cell that a no-slip face's gradient ghost reads; prev(): the cell's previous-stage state.
+template <class Ghost, class Prev>
+__device__ __forceinline__ void tile_gradient(const TileView& v, const Consts<float>& k, int gI, bool squeeze, bool lim_prev,
+                                              bool init_prims, bool stage0, const float4& mom, const Q4<float>& gpx,
+                                              const Q4<float>& gpy, Ghost ghost, Prev prev, Q4<float>& gx, Q4<float>& gy) {
+    const Q4<float> qc = v.cq[gI];
+    // LSQ sums (Q(c2) - Q(c1)) * (dxj, dyj) over the cell's faces and, for the squeeze limiter, the
+    // extremes over the neighbours of Q(n) - Q(c) (= the bounds Qmax - Q, Qmin - Q of squeeze.cpp:
+    // rounding is monotone, so the extreme difference is the difference of the extreme) and over the
+    // faces of gprev . (face centre - centre), the previous face value's part that varies by face
+    // (its base Qprev - Q is added after the loop, again exactly for the extremes)
+    float sx[4] = {0.f, 0.f, 0.f, 0.f}, sy[4] = {0.f, 0.f, 0.f, 0.f};
+    float dmin[4], dmax[4], tmin[4], tmax[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        dmin[j] = 0.f; dmax[j] = 0.f;
+        tmin[j] = 3.0e38f; tmax[j] = -3.0e38f;
+    }
+    // bit 15 of the end offset: the cell has a boundary face; the others' loop has no boundary
+    // branches
+    const uint32_t o1 = v.off[gI + 1];
+    const int e0 = v.off[gI] & 0x7FFF, e1 = (int)(o1 & 0x7FFFu);
+    auto face_loop = [&](auto interior) {
+        constexpr bool INTERIOR = decltype(interior)::value;
+        for (int e = e0; e < e1; e++) {
+            const uint32_t ent = v.ent[e];
+            const int r = (int)((ent & 0xFFFFu) >> 1), side = (int)(ent & 1u);
+            const int so = (int)(int16_t)(ent >> 16);   // the face's other cell (or BC code)
+            const float4 dd = v.d[r];
+            const float d1x = dd.x, d1y = dd.y, d2x = dd.z, d2y = dd.w;
+            float d[4];
+            if (INTERIOR || so >= 0) {
+                const Q4<float> qn = v.cq[so];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    d[j] = fs(qn.p[j], qc.p[j]);
+                    if (squeeze) { dmin[j] = fminf(dmin[j], d[j]); dmax[j] = fmaxf(dmax[j], d[j]); }
+                }
+            } else if (so == -1) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) d[j] = fs(k.q_inf[j], qc.p[j]);
+            } else if (so == -2 || so == -4) {
+                float rho, u, vv, P, yr, gq[4];
+                if (so == -2) {   // slip wall: the cell velocity reflected (cell_gradient.cpp:43-55)
+                    if (init_prims) { rho = k.rho_inf; u = k.u_inf; vv = k.v_inf; P = k.P_inf; }
+                    else tprims(qc.p, k, rho, u, vv, P, yr);
+                    const float fnx = v.nx[r], fny = v.ny[r];
+                    const float vn2 = fm(2.0f, mm(u, fnx, vv, fny));
+                    tcons(rho, ff(-vn2, fnx, u), ff(-vn2, fny, vv), P, k, gq);
+                } else if (stage0) {   // no-slip: cell `face id`'s state, velocity negated (:62-73)
+                    if (init_prims) { rho = k.rho_inf; u = k.u_inf; vv = k.v_inf; P = k.P_inf; }
+                    else { const Q4<float> qq = ghost(r); tprims(qq.p, k, rho, u, vv, P, yr); }
+                    tcons(rho, -u, -vv, P, k, gq);
+                } else {
+                    const Q4<float> qq = ghost(r);
+                    tghost_noslip(qq.p, k, gq);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) d[j] = fs(gq[j], qc.p[j]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++) d[j] = 0.f;
+            }
+            // LSQ displacement c1 -> c2 (or ghost), times Q(c2) - Q(c1): for a c2-side cell the
+            // difference above is Q(c1) - Q(c2), so the displacement's sign is flipped instead
+            const float fx = side ? fs(d2x, d1x) : fs(d1x, d2x), fy = side ? fs(d2y, d1y) : fs(d1y, d2y);
+            const float ox = side ? d2x : d1x, oy = side ? d2y : d1y;   // face centre - this cell
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                sx[j] = ff(d[j], fx, sx[j]);
+                sy[j] = ff(d[j], fy, sy[j]);
+                if (lim_prev) {
+                    const float x = mm(gpx.p[j], ox, gpy.p[j], oy);
+                    tmin[j] = fminf(tmin[j], x);
+                    tmax[j] = fmaxf(tmax[j], x);
+                }
+            }
+        }
+    };
+    // one loop per warp: the general one if any of its cells has a boundary face (a warp running
+    // both would take the sum of the two)
+    if (__any_sync(__activemask(), (o1 & 0x8000u) != 0)) face_loop(std::false_type{});
+    else face_loop(std::true_type{});
+    const float ixx = mom.x, iyy = mom.y, ixy = mom.z;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        gx.p[j] = mm(sx[j], iyy, -sy[j], ixy);
+        gy.p[j] = mm(sy[j], ixx, -sx[j], ixy);
+    }
+    if (squeeze) {
+        // squeeze (squeeze.cpp:68-141): phi = the smallest (bound - Q) / (face value - Q) over the
+        // faces whose previous face value leaves [Qmin, Qmax]; as x -> (bound - Q) / x is monotone
+        // on either side of zero, that is the quotient at the extreme t
+        Q4<float> qp;
+        if (lim_prev) qp = prev();
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float up = dmax[j], dn = dmin[j];
+            // t = (previous face value) - Q: its base plus the extremes above; -101 is the fresh
+            // face history's value
+            const float base = lim_prev ? fs(qp.p[j], qc.p[j]) : fs(-101.0f, qc.p[j]);
+            const float thi = lim_prev ? fa(base, tmax[j]) : base, tlo = lim_prev ? fa(base, tmin[j]) : base;
+            float phi = 1.0f;
+            if (thi > up) phi = fminf(phi, up / thi);
+            if (tlo < dn) phi = fminf(phi, dn / tlo);
+            gx.p[j] = fm(gx.p[j], phi);
+            gy.p[j] = fm(gy.p[j], phi);
+        }
+    }
+}
+
+// Flux of one face of a core cell (record r): V*A - F*A to w_t[r] and, on an iteration's last
+// stage, its spectral term to w_sp[r].  (w_t and w_sp may be the record's own displacement and
+// normal-x rows: both are read before they are written.)  INTERIOR: the record joins two cells, so
+// the boundary branches go and both sides' reconstructions can be scheduled together.
+template <bool INTERIOR>
+__device__ __forceinline__ void tile_flux(const TileView& v, const Consts<float>& k, int r, bool order2, bool visc,
+                                          bool init_prims, bool last, float4* w_t, float* w_sp) {
+    const Q4<float>* cq = v.cq;
+    const Q4<float>* cg = v.cg;
+    const uint32_t sl = v.sl[r];
+    const int s1 = (int)(sl & 0xFFFFu), s2 = (int)(int16_t)(sl >> 16);
+    const float4 dd = v.d[r];
+    const float d1x = dd.x, d1y = dd.y, d2x = dd.z, d2y = dd.w;
+    const float fnx = v.nx[r], fny = v.ny[r];
+    const float mxf = -fny, myf = fnx;   // unit tangent p1 -> p2
+    // face states; for NS also the face-average tangential derivative m.(grad Q1 + grad Q2)/2,
+    // the difference Q2 - Q1 and c1's velocity, so the cell states and gradients die early
+    float L[4], Rq[4], dm[4], dq[4];
+    float cu = 0.f, cv = 0.f;
+    {
+        const Q4<float> q1 = cq[s1];
+        Q4<float> g1x, g1y;
+        if (order2) { g1x = cg[2 * s1]; g1y = cg[2 * s1 + 1]; }
+        else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) { g1x.p[j] = 0.f; g1y.p[j] = 0.f; }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            L[j] = ff(g1y.p[j], d1y, ff(g1x.p[j], d1x, q1.p[j]));
+            dm[j] = mm(g1y.p[j], myf, g1x.p[j], mxf);
+            dq[j] = -q1.p[j];
+        }
+        if (!INTERIOR && visc && s2 == -4) {
+            if (init_prims) { cu = k.u_inf; cv = k.v_inf; }
+            else { const float yq = 1.0f / q1.p[0]; cu = fm(q1.p[1], yq); cv = fm(q1.p[2], yq); }
+        }
+    }
+    float lrho, lu, lv, lP, ly;
+    tprims(L, k, lrho, lu, lv, lP, ly);
+    if (INTERIOR || s2 >= 0) {
+        const Q4<float> q2 = cq[s2];
+        Q4<float> g2x, g2y;
+        if (order2) { g2x = cg[2 * s2]; g2y = cg[2 * s2 + 1]; }
+        else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) { g2x.p[j] = 0.f; g2y.p[j] = 0.f; }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            Rq[j] = ff(g2y.p[j], d2y, ff(g2x.p[j], d2x, q2.p[j]));
+            dm[j] = fm(0.5f, ff(g2y.p[j], myf, ff(g2x.p[j], mxf, dm[j])));
+            dq[j] = fa(dq[j], q2.p[j]);
+        }
+    } else if (s2 == -1) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) Rq[j] = k.q_inf[j];
+    } else if (s2 == -2) {
+        const float vn2 = fm(2.0f, mm(lu, fnx, lv, fny));
+        tcons(lrho, ff(-vn2, fnx, lu), ff(-vn2, fny, lv), lP, k, Rq);
+    } else if (s2 == -3) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) Rq[j] = L[j];
+    } else {
+        tghost_noslip(L, k, Rq);
+    }
+    const float A = v.A[r];
+    const float lc = sqrtf(fm(fm(k.gamma, lP), ly));
+    float rrho, ru, rv, rP, ry;
+    tprims(Rq, k, rrho, ru, rv, rP, ry);
+    const float rc = sqrtf(fm(fm(k.gamma, rP), ry));
+    const float vn1 = mm(lu, fnx, lv, fny), vn2 = mm(ru, fnx, rv, fny);
+    const float vna = fm(0.5f, fa(vn1, vn2)), ca = fm(0.5f, fa(lc, rc));
+    const float sp = fa(fabsf(vna), ca);
+    const float lam = fm(0.5f, sp);
+    float Fr[4];
+    if (k.roe) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) Fr[j] = -101.0f;
+    } else {
+        // F(L) + F(R)
+        const float lE = fa(L[3], lP);
+        const float rE = fa(Rq[3], rP);
+        const float X[4] = {
+            mm(lrho, vn1, rrho, vn2),
+            fa(mm(fm(lrho, lu), vn1, lP, fnx), mm(fm(rrho, ru), vn2, rP, fnx)),
+            fa(mm(fm(lrho, lv), vn1, lP, fny), mm(fm(rrho, rv), vn2, rP, fny)),
+            mm(vn1, lE, vn2, rE)};
+#pragma unroll
+        for (int j = 0; j < 4; j++) Fr[j] = mm(0.5f, X[j], -lam, fs(Rq[j], L[j]));
+    }
+    float V[4] = {0.f, 0.f, 0.f, 0.f};
+    if (visc) {   // first order never adds the viscous flux (res.cpp:27-29,50-53)
+        float S[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) S[j] = fa(L[j], Rq[j]);
+        const float arho = fm(0.5f, S[0]), ya = 1.0f / arho;
+        const float au = fm(fm(0.5f, S[1]), ya), av = fm(fm(0.5f, S[2]), ya);
+        const float ke = mm(au, au, av, av);
+        const float aP = fm(mm(0.5f, S[3], -fm(0.5f, arho), ke), k.gm1);
+        float ux = 0.f, uy = 0.f, vx = 0.f, vy = 0.f, Px = 0.f, Py = 0.f, rx = 0.f, rly = 0.f;
+        bool have = true;
+        if (INTERIOR || s2 >= 0) {
+            // l: unit vector c1 -> c2 (the LSQ displacement d1 - d2)
+            const float tx = fs(d1x, d2x), ty = fs(d1y, d2y);
+            const float yd = rsqrtf(mm(tx, tx, ty, ty));
+            const float lxf = fm(tx, yd), lyf = fm(ty, yd);
+            float dl[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) dl[j] = ff(dq[j], yd, dm[j]);   // reconstruction.cpp:138-146: l for both terms
+            rx = fm(dl[0], lxf);
+            const float rxu = fm(rx, au), rxv = fm(rx, av);
+            ux = mm(dl[1], lxf, -rxu, ya);
+            vx = mm(dl[2], lxf, -rxv, ya);
+            rly = fm(dl[0], lyf);
+            const float ryu = fm(rly, au);
+            uy = mm(dl[1], lyf, -ryu, ya);
+            vy = mm(dl[2], lyf, -ryu, ya);   // reconstruction.cpp:155 uses u
+            Px = fm(k.gm1, ff(-arho, mm(au, ux, av, vx), mm(dl[3], lxf, -fm(0.5f, rx), ke)));
+            Py = fm(k.gm1, ff(-arho, mm(au, uy, av, vy), mm(dl[3], lyf, -fm(0.5f, rly), ke)));
+        } else if (s2 == -4) {
+            const float ydn = rsqrtf(mm(d1x, d1x, d1y, d1y));
+            const float dudn = fm(-cu, ydn), dvdn = fm(-cv, ydn);
+            ux = fm(dudn, fnx); uy = fm(dudn, fny);
+            vx = fm(dvdn, fnx); vy = fm(dvdn, fny);
+        } else if (s2 == -2) {
+            have = false;   // SLIP_WALL with NS: tau and grad T stay zero (:104-106)
+        }
+        if (have) {
+            const float div = fa(ux, vy), mu2 = fm(2.0f, k.mu), third = 1.0f / 3.0f;
+            const float txx = fm(mu2, ff(-div, third, ux));
+            const float tyy = fm(mu2, ff(-div, third, vy));
+            const float txy = fm(k.mu, fa(uy, vx));
+            const float yden = 1.0f / fm(fm(k.R, arho), arho);
+            const float dTx = fm(mm(Px, arho, -rx, aP), yden);
+            const float dTy = fm(mm(Py, arho, -rly, aP), yden);
+            V[1] = mm(txy, fny, txx, fnx);
+            V[2] = mm(txy, fnx, tyy, fny);
+            V[3] = mm(fnx, ff(k.k, dTx, mm(av, txy, au, txx)), fny,
+                      ff(k.k, dTy, mm(au, txy, av, tyy)));
+        }
+    }
+    w_t[r] = make_float4(fm(fs(V[0], Fr[0]), A), fm(fs(V[1], Fr[1]), A), fm(fs(V[2], Fr[2]), A), fm(fs(V[3], Fr[3]), A));
+    if (last) w_sp[r] = k.roe ? fm(fa(fabsf(k.vn0), k.c0), A) : fm(sp, A);
+}
+
+// Residual of core cell c (res.cpp:74-109): its faces' contributions in ascending original face id,
+// over its volume (yv = 1/vol); on the last stage its spectral terms' sum too.
+__device__ __forceinline__ void tile_residual(const TileView& v, int c, const float4* w_t, const float* w_sp, bool last,
+                                              float yv, float r4[4], float& snext) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) r4[j] = 0.f;
+    const int e0 = v.off[c] & 0x7FFF, e1 = v.off[c + 1] & 0x7FFF;
+    for (int e = e0; e < e1; e++) {
+        const uint32_t ent = v.ent[e];
+        const int r = (int)((ent & 0xFFFFu) >> 1), side = (int)(ent & 1u);
+        const float4 tv = w_t[r];
+        r4[0] = fa(r4[0], neg_if(tv.x, side));
+        r4[1] = fa(r4[1], neg_if(tv.y, side));
+        r4[2] = fa(r4[2], neg_if(tv.z, side));
+        r4[3] = fa(r4[3], neg_if(tv.w, side));
+        if (last) snext = fa(snext, w_sp[r]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) r4[j] = fm(r4[j], yv);
+}
+
+// The SSP-RK3 stage (ssp_rk3.cpp:50-77) in the compensated delta form: dn the new increment (first
+// two stages), out the new state, lo the base state's compensation (updated by the last stage).
+__device__ __forceinline__ void stage_combine(int stage, float dtc, const float r4[4], const Q4<float>& qn,
+                                              const Q4<float>& dprev, Q4<float>& lo, Q4<float>& dn, Q4<float>& out) {
+    if (stage == 0) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            dn.p[j] = fm(dtc, r4[j]);
+            out.p[j] = fa(qn.p[j], dn.p[j]);
+        }
+    } else if (stage == 1) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            dn.p[j] = mm(0.25f, dprev.p[j], fm(0.25f, dtc), r4[j]);
+            out.p[j] = fa(qn.p[j], dn.p[j]);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float inc = mm(2.0f / 3.0f, dprev.p[j], fm(2.0f / 3.0f, dtc), r4[j]);
+            float s, err;
+            two_sum(qn.p[j], fa(lo.p[j], inc), s, err);
+            out.p[j] = s;
+            lo.p[j] = err;
+        }
+    }
 }
 
 template <int STAGE>
@@ -293,266 +641,36 @@ __global__ void __launch_bounds__(kTileCore, 3) k_tstage(TArgs a) {
         const bool order2 = tp.order2 != 0, ns = tp.ns != 0;
         const bool fresh = STAGE == 0 && tp.fresh != 0, init_prims = STAGE == 0 && tp.init_prims != 0;
         const bool squeeze = tp.squeeze != 0;
-        const uint32_t* __restrict__ r_sl = srec;
-        const float4* __restrict__ r_d = reinterpret_cast<const float4*>(srec + nrp);
-        const float* __restrict__ r_nx = reinterpret_cast<const float*>(srec + 5 * nrp);
-        const float* __restrict__ r_ny = reinterpret_cast<const float*>(srec + 5 * nrp + ngp);
-        const float* __restrict__ r_A = reinterpret_cast<const float*>(srec + 5 * nrp + 2 * ngp);
-        const uint16_t* __restrict__ c_off = scsr;
-        const uint32_t* __restrict__ c_ent = reinterpret_cast<const uint32_t*>(scsr + td.noff);
+        const TileView tv{srec, reinterpret_cast<const float4*>(srec + nrp),
+                          reinterpret_cast<const float*>(srec + 5 * nrp),
+                          reinterpret_cast<const float*>(srec + 5 * nrp + ngp),
+                          reinterpret_cast<const float*>(srec + 5 * nrp + 2 * ngp),
+                          scsr, reinterpret_cast<const uint32_t*>(scsr + td.noff), cq, cg};
 
         // ---- grad: the limited LSQ gradient of one core or ring-1 cell (local slot gI)
         auto grad_cell = [&](int gI) {
-            {
-                const int gid = gI < ncore ? c0 + gI : cbase + shalo[gI - ncore];
-                const bool lim_prev = squeeze && !fresh;
-                // requested first: used only after the loop over the cell's faces
-                const float4 mom = a.lsq[gid];
-                Q4<float> gpx, gpy;
-                if (lim_prev) { gpx = Gprev[2 * (size_t)gid]; gpy = Gprev[2 * (size_t)gid + 1]; }
-                const Q4<float> qc = cq[gI];
-                // LSQ sums (Q(c2) - Q(c1)) * (dxj, dyj) over the cell's faces and, for the squeeze
-                // limiter, the extremes over the neighbours of Q(n) - Q(c) (= the bounds Qmax - Q,
-                // Qmin - Q of squeeze.cpp: rounding is monotone, so the extreme difference is the
-                // difference of the extreme) and over the faces of gprev . (face centre - centre), the
-                // previous face value's part that varies by face (its base Qprev - Q is added after
-                // the loop, again exactly for the extremes)
-                float sx[4] = {0.f, 0.f, 0.f, 0.f}, sy[4] = {0.f, 0.f, 0.f, 0.f};
-                float dmin[4], dmax[4], tmin[4], tmax[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    dmin[j] = 0.f; dmax[j] = 0.f;
-                    tmin[j] = 3.0e38f; tmax[j] = -3.0e38f;
-                }
-                // bit 15 of the end offset: the cell has a boundary face; the others' loop has no
-                // boundary branches
-                const uint32_t o1 = c_off[gI + 1];
-                const int e0 = c_off[gI] & 0x7FFF, e1 = (int)(o1 & 0x7FFFu);
-                auto face_loop = [&](auto interior) {
-                    constexpr bool INTERIOR = decltype(interior)::value;
-                    for (int e = e0; e < e1; e++) {
-                        const uint32_t ent = c_ent[e];
-                        const int r = (int)((ent & 0xFFFFu) >> 1), side = (int)(ent & 1u);
-                        const int so = (int)(int16_t)(ent >> 16);   // the face's other cell (or BC code)
-                        const float4 dd = r_d[r];
-                        const float d1x = dd.x, d1y = dd.y, d2x = dd.z, d2y = dd.w;
-                        float d[4];
-                        if (INTERIOR || so >= 0) {
-                            const Q4<float> qn = cq[so];
-    #pragma unroll
-                            for (int j = 0; j < 4; j++) {
-                                d[j] = qn.p[j] - qc.p[j];
-                                if (squeeze) { dmin[j] = fminf(dmin[j], d[j]); dmax[j] = fmaxf(dmax[j], d[j]); }
-                            }
-                        } else if (so == -1) {
-    #pragma unroll
-                            for (int j = 0; j < 4; j++) d[j] = k.q_inf[j] - qc.p[j];
-                        } else if (so == -2 || so == -4) {
-                            float rho, u, v, P, yr;
-                            if (init_prims) { rho = k.rho_inf; u = k.u_inf; v = k.v_inf; P = k.P_inf; }
-                            else if (so == -2) tprims(qc.p, k, rho, u, v, P, yr);
-                            else {
-                                const Q4<float> qq = Qin[cbase + a.qcell[td.rbase + r]];
-                                tprims(qq.p, k, rho, u, v, P, yr);
-                            }
-                            float gq[4];
-                            if (so == -2) {   // slip wall: the cell velocity reflected (cell_gradient.cpp:43-55)
-                                const float fnx = r_nx[r], fny = r_ny[r];
-                                const float vn = u * fnx + v * fny;
-                                cons(rho, u - 2.0f * vn * fnx, v - 2.0f * vn * fny, P, k, gq);
-                            } else {          // no-slip: cell `face id`'s state, velocity negated (:62-73)
-                                cons(rho, -u, -v, P, k, gq);
-                            }
-    #pragma unroll
-                            for (int j = 0; j < 4; j++) d[j] = gq[j] - qc.p[j];
-                        } else {
-    #pragma unroll
-                            for (int j = 0; j < 4; j++) d[j] = 0.f;
-                        }
-                        // LSQ displacement c1 -> c2 (or ghost), times Q(c2) - Q(c1): for a c2-side cell the
-                        // difference above is Q(c1) - Q(c2), so the displacement's sign is flipped instead
-                        const float fx = side ? d2x - d1x : d1x - d2x, fy = side ? d2y - d1y : d1y - d2y;
-                        const float ox = side ? d2x : d1x, oy = side ? d2y : d1y;   // face centre - this cell
-    #pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            sx[j] += d[j] * fx;
-                            sy[j] += d[j] * fy;
-                            if (lim_prev) {
-                                const float x = gpx.p[j] * ox + gpy.p[j] * oy;
-                                tmin[j] = fminf(tmin[j], x);
-                                tmax[j] = fmaxf(tmax[j], x);
-                            }
-                        }
-                    }
-                };
-                // one loop per warp: the general one if any of its cells has a boundary face (a warp
-                // running both would take the sum of the two)
-                if (__any_sync(__activemask(), (o1 & 0x8000u) != 0)) face_loop(std::false_type{});
-                else face_loop(std::true_type{});
-                const float ixx = mom.x, iyy = mom.y, ixy = mom.z;
-                Q4<float> gx, gy;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    gx.p[j] = sx[j] * iyy - sy[j] * ixy;
-                    gy.p[j] = sy[j] * ixx - sx[j] * ixy;
-                }
-                if (squeeze) {
-                    // squeeze (squeeze.cpp:68-141): phi = the smallest (bound - Q) / (face value - Q) over
-                    // the faces whose previous face value leaves [Qmin, Qmax]; as x -> (bound - Q) / x is
-                    // monotone on either side of zero, that is the quotient at the extreme t
-                    Q4<float> qp;
-                    if (lim_prev) qp = Qprev[gid];
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const float up = dmax[j], dn = dmin[j];
-                        // t = (previous face value) - Q: its base plus the extremes above; -101 is the
-                        // fresh face history's value
-                        const float base = lim_prev ? qp.p[j] - qc.p[j] : -101.0f - qc.p[j];
-                        const float thi = lim_prev ? base + tmax[j] : base, tlo = lim_prev ? base + tmin[j] : base;
-                        float phi = 1.0f;
-                        if (thi > up) phi = fminf(phi, up / thi);
-                        if (tlo < dn) phi = fminf(phi, dn / tlo);
-                        gx.p[j] *= phi;
-                        gy.p[j] *= phi;
-                    }
-                }
-                cg[2 * gI] = gx;
-                cg[2 * gI + 1] = gy;
-                if (gI < ncore) { Gout[2 * (size_t)gid] = gx; Gout[2 * (size_t)gid + 1] = gy; }
-            }
+            const int gid = gI < ncore ? c0 + gI : cbase + shalo[gI - ncore];
+            const bool lim_prev = squeeze && !fresh;
+            // requested first: used only after the loop over the cell's faces
+            const float4 mom = a.lsq[gid];
+            Q4<float> gpx, gpy;
+            if (lim_prev) { gpx = Gprev[2 * (size_t)gid]; gpy = Gprev[2 * (size_t)gid + 1]; }
+            Q4<float> gx, gy;
+            tile_gradient(tv, k, gI, squeeze, lim_prev, init_prims, STAGE == 0, mom, gpx, gpy,
+                          [&](int r) { return Qin[cbase + a.qcell[td.rbase + r]]; }, [&] { return Qprev[gid]; }, gx, gy);
+            cg[2 * gI] = gx;
+            cg[2 * gI + 1] = gy;
+            if (gI < ncore) { Gout[2 * (size_t)gid] = gx; Gout[2 * (size_t)gid + 1] = gy; }
         };
 
         // ---- flux of one face of a core cell (record r); V*A - F*A replaces its displacement row
         // and the spectral term its normal's x
-            float4* w_t = reinterpret_cast<float4*>(srec + nrp);
-            float* w_sp = reinterpret_cast<float*>(srec + 5 * nrp);
-            const bool visc = ns && order2;   // first order never adds the viscous flux (res.cpp:27-29,50-53)
-            // INTERIOR (a compile-time tag): the record joins two cells, so the boundary branches go
-            // and both sides' reconstructions can be scheduled together
-            auto flux_rec = [&](int r, auto interior) {
-                constexpr bool INTERIOR = decltype(interior)::value;
-                const uint32_t sl = r_sl[r];
-                const int s1 = (int)(sl & 0xFFFFu), s2 = (int)(int16_t)(sl >> 16);
-                const float4 dd = r_d[r];
-                const float d1x = dd.x, d1y = dd.y, d2x = dd.z, d2y = dd.w;
-                const float fnx = r_nx[r], fny = r_ny[r];
-                const float mxf = -fny, myf = fnx;   // unit tangent p1 -> p2
-                // face states; for NS also the face-average tangential derivative m.(grad Q1 + grad Q2)/2,
-                // the difference Q2 - Q1 and c1's velocity, so the cell states and gradients die early
-                float L[4], Rq[4], dm[4], dq[4];
-                float cu = 0.f, cv = 0.f;
-                {
-                    const Q4<float> q1 = cq[s1];
-                    Q4<float> g1x, g1y;
-                    if (order2) { g1x = cg[2 * s1]; g1y = cg[2 * s1 + 1]; }
-                    else {
-#pragma unroll
-                        for (int j = 0; j < 4; j++) { g1x.p[j] = 0.f; g1y.p[j] = 0.f; }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        L[j] = q1.p[j] + g1x.p[j] * d1x + g1y.p[j] * d1y;
-                        dm[j] = g1x.p[j] * mxf + g1y.p[j] * myf;
-                        dq[j] = -q1.p[j];
-                    }
-                    if (!INTERIOR && visc && s2 == -4) {
-                        if (init_prims) { cu = k.u_inf; cv = k.v_inf; }
-                        else { const float yq = 1.0f / q1.p[0]; cu = q1.p[1] * yq; cv = q1.p[2] * yq; }
-                    }
-                }
-                float lrho, lu, lv, lP, ly;
-                tprims(L, k, lrho, lu, lv, lP, ly);
-                if (INTERIOR || s2 >= 0) {
-                    const Q4<float> q2 = cq[s2];
-                    Q4<float> g2x, g2y;
-                    if (order2) { g2x = cg[2 * s2]; g2y = cg[2 * s2 + 1]; }
-                    else {
-#pragma unroll
-                        for (int j = 0; j < 4; j++) { g2x.p[j] = 0.f; g2y.p[j] = 0.f; }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        Rq[j] = q2.p[j] + g2x.p[j] * d2x + g2y.p[j] * d2y;
-                        dm[j] = 0.5f * (dm[j] + g2x.p[j] * mxf + g2y.p[j] * myf);
-                        dq[j] += q2.p[j];
-                    }
-                } else if (s2 == -1) {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) Rq[j] = k.q_inf[j];
-                } else if (s2 == -2) {
-                    const float vn = lu * fnx + lv * fny;
-                    cons(lrho, lu - 2.0f * vn * fnx, lv - 2.0f * vn * fny, lP, k, Rq);
-                } else if (s2 == -3) {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) Rq[j] = L[j];
-                } else {
-                    cons(lrho, -lu, -lv, lP, k, Rq);
-                }
-                const float A = r_A[r];
-                const float lc = sqrtf(k.gamma * lP * ly);
-                float rrho, ru, rv, rP, ry;
-                tprims(Rq, k, rrho, ru, rv, rP, ry);
-                const float rc = sqrtf(k.gamma * rP * ry);
-                const float vn1 = lu * fnx + lv * fny, vn2 = ru * fnx + rv * fny;
-                const float vna = 0.5f * (vn1 + vn2), ca = 0.5f * (lc + rc);
-                const float lam = 0.5f * (fabsf(vna) + ca);
-                float Fr[4];
-                {
-                    const float F1[4] = {lrho * vn1, lrho * lu * vn1 + lP * fnx, lrho * lv * vn1 + lP * fny, vn1 * (L[3] + lP)};
-                    const float F2[4] = {rrho * vn2, rrho * ru * vn2 + rP * fnx, rrho * rv * vn2 + rP * fny, vn2 * (Rq[3] + rP)};
-#pragma unroll
-                    for (int j = 0; j < 4; j++) Fr[j] = k.roe ? -101.0f : 0.5f * (F1[j] + F2[j]) - lam * (Rq[j] - L[j]);
-                }
-                float V[4] = {0.f, 0.f, 0.f, 0.f};
-                if (visc) {
-                    float Aq[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++) Aq[j] = 0.5f * (L[j] + Rq[j]);
-                    float arho, au, av, aP, ya;
-                    tprims(Aq, k, arho, au, av, aP, ya);
-                    float ux = 0.f, uy = 0.f, vx = 0.f, vy = 0.f, Px = 0.f, Py = 0.f, rx = 0.f, rly = 0.f;
-                    bool have = true;
-                    if (INTERIOR || s2 >= 0) {
-                        // l: unit vector c1 -> c2 (the LSQ displacement d1 - d2)
-                        const float tx = d1x - d2x, ty = d1y - d2y;
-                        const float yd = rsqrtf(tx * tx + ty * ty);
-                        const float lxf = tx * yd, lyf = ty * yd;
-                        float dQx[4], dQy[4];
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            const float dl = dq[j] * yd + dm[j];   // reconstruction.cpp:138-146: l for both terms
-                            dQy[j] = dl * lyf;
-                            dQx[j] = dl * lxf;
-                        }
-                        rx = dQx[0];
-                        ux = dQx[1] - rx * au * ya;
-                        vx = dQx[2] - rx * av * ya;
-                        rly = dQy[0];
-                        uy = dQy[1] - rly * au * ya;
-                        vy = dQy[2] - rly * au * ya;   // reconstruction.cpp:155 uses u
-                        Px = k.gm1 * (dQx[3] - 0.5f * rx * (au * au + av * av) - arho * (au * ux + av * vx));
-                        Py = k.gm1 * (dQy[3] - 0.5f * rly * (au * au + av * av) - arho * (au * uy + av * vy));
-                    } else if (s2 == -4) {
-                        const float ydn = rsqrtf(d1x * d1x + d1y * d1y);
-                        const float dudn = -cu * ydn, dvdn = -cv * ydn;
-                        ux = dudn * fnx; uy = dudn * fny;
-                        vx = dvdn * fnx; vy = dvdn * fny;
-                    } else if (s2 == -2) {
-                        have = false;   // SLIP_WALL with NS: tau and grad T stay zero (:104-106)
-                    }
-                    if (have) {
-                        const float third = (ux + vy) * (1.0f / 3.0f);
-                        const float txx = 2.0f * k.mu * (ux - third), txy = k.mu * (uy + vx), tyy = 2.0f * k.mu * (vy - third);
-                        const float yden = 1.0f / (k.R * arho * arho);
-                        const float dTx = (Px * arho - rx * aP) * yden, dTy = (Py * arho - rly * aP) * yden;
-                        V[1] = txx * fnx + txy * fny;
-                        V[2] = txy * fnx + tyy * fny;
-                        V[3] = fnx * (au * txx + av * txy + k.k * dTx) + fny * (au * txy + av * tyy + k.k * dTy);
-                    }
-                }
-                w_t[r] = make_float4((V[0] - Fr[0]) * A, (V[1] - Fr[1]) * A, (V[2] - Fr[2]) * A, (V[3] - Fr[3]) * A);
-                if (STAGE == 2) w_sp[r] = k.roe ? (fabsf(k.vn0) + k.c0) * A : (fabsf(vna) + ca) * A;
-            };
+        float4* w_t = reinterpret_cast<float4*>(srec + nrp);
+        float* w_sp = reinterpret_cast<float*>(srec + 5 * nrp);
+        const bool visc = ns && order2;
+        auto flux_rec = [&](int r, auto interior) {
+            tile_flux<decltype(interior)::value>(tv, k, r, order2, visc, init_prims, STAGE == 2, w_t, w_sp);
+        };
 
         // ---- schedule: core-cell gradients; then the ring-1 gradients on the first warps while the
         // other warps take the fluxes of faces between two core cells (they need core gradients
@@ -613,8 +731,6 @@ __global__ void __launch_bounds__(kTileCore, 3) k_tstage(TArgs a) {
         float r2[4] = {0.f, 0.f, 0.f, 0.f};
         if (tid < ncore) {
             const int c = tid, gid = c0 + c;
-            const float4* tt = reinterpret_cast<const float4*>(srec + nrp);
-            const float* sp = reinterpret_cast<const float*>(srec + 5 * nrp);
             // the stage's cell data, requested before the gather
             const float yv = a.rvol[gid];
             float dtc = 0.f, sc = 0.f, vc = 0.f;
@@ -624,45 +740,22 @@ __global__ void __launch_bounds__(kTileCore, 3) k_tstage(TArgs a) {
             if (STAGE == 0) qn = cq[c];
             else { qn = a.Q[0][gid]; dprev = a.D[gid]; }
             if (STAGE == 2) lo = a.Qlo[gid];
-            float r4[4] = {0.f, 0.f, 0.f, 0.f};
-            const int e0 = c_off[c] & 0x7FFF, e1 = c_off[c + 1] & 0x7FFF;
-            for (int e = e0; e < e1; e++) {
-                const uint32_t ent = c_ent[e];
-                const int r = (int)((ent & 0xFFFFu) >> 1), side = (int)(ent & 1u);
-                const float4 tv = tt[r];
-                r4[0] += neg_if(tv.x, side);
-                r4[1] += neg_if(tv.y, side);
-                r4[2] += neg_if(tv.z, side);
-                r4[3] += neg_if(tv.w, side);
-                if (STAGE == 2) snext += sp[r];
-            }
-#pragma unroll
-            for (int j = 0; j < 4; j++) r4[j] *= yv;
+            float r4[4];
+            tile_residual(tv, c, w_t, w_sp, STAGE == 2, yv, r4, snext);
             if (a.R && (a.store_r || STAGE == 2)) { Q4<float> rr; for (int j = 0; j < 4; j++) rr.p[j] = r4[j]; a.R[gid] = rr; }
             if (STAGE == 0) {
-                dtc = (k.two_cfl * vc) / (tp.global_dt ? a.smax[td.sid] : sc);
+                dtc = fm(k.two_cfl, vc) / (tp.global_dt ? a.smax[td.sid] : sc);
                 a.dt[gid] = dtc;
             }
             Q4<float> out, dn;
+            stage_combine(STAGE, dtc, r4, qn, dprev, lo, dn, out);
             if (STAGE == 0) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) { dn.p[j] = dtc * r4[j]; out.p[j] = qn.p[j] + dn.p[j]; }
                 a.D[gid] = dn;
                 a.Q[1][gid] = out;
             } else if (STAGE == 1) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) { dn.p[j] = 0.25f * dprev.p[j] + 0.25f * dtc * r4[j]; out.p[j] = qn.p[j] + dn.p[j]; }
                 a.D[gid] = dn;
                 a.Q[2][gid] = out;
             } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float inc = (2.0f / 3.0f) * dprev.p[j] + (2.0f / 3.0f) * dtc * r4[j];
-                    float s, err;
-                    two_sum(qn.p[j], lo.p[j] + inc, s, err);
-                    out.p[j] = s;
-                    lo.p[j] = err;
-                }
                 a.Q[0][gid] = out;
                 a.Qlo[gid] = lo;
                 a.S[gid] = snext;
@@ -694,6 +787,232 @@ __global__ void __launch_bounds__(kTileCore, 3) k_tstage(TArgs a) {
             red_sid = td.sid;
         }
         __syncthreads();
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// Whole iterations in one launch, for solves whose tiles all fit on the GPU at once (one tile per
+// CTA, a cooperative launch): a tile's records, csr and halo list are copied to shared memory once
+// per launch, its states and limited gradients stay there from stage to stage, its cells' RK data in
+// registers; the tiles exchange only their new states, through L2, with one grid barrier per stage.
+// Such a solve is bound by latency, not by any unit: with a stage kernel per stage it spends ~15 us a
+// stage on the launch, the tile's block copies and a 256-cell tile's passes on a third of the SMs.
+// Here a stage is the barrier and the ring gather (~1.5 us), one round of gradients and fluxes and
+// the update: 12k-cell NS cylinder 45.2 -> 16.7 us per iteration, 50k Euler polygons 42.7 -> 20.0, 512
+// quads 26 -> 11.1.  What the passes read every stage (LSQ moments, previous states) is kept in shared
+// memory too, since the barrier's acquire empties L1 (the 12k-cell cylinder: 19.8 -> 16.7
+// us, with a barrier that has no fences beyond its release and acquire).  MINB 2 has the registers to run without spills; MINB 3 (144 B of spills) takes
+// the solves whose tiles do not fit two to an SM.
+struct TIter {
+    int iterations;
+    unsigned bar0;             // the barrier's value when the launch starts
+    unsigned* bar;             // arrivals so far (monotone, wraps)
+    int o_csr, o_halo, o_cq, o_cg, o_t, o_sp, o_qp, o_lsq;   // shared-memory regions (bytes; the record block is at 0)
+    int max_rec, max_csr, max_halo, max_cells, max_grad, max_flux;   // and what they hold (TileLayout's maxima)
+};
+
+// A state from L2 (the SM's own L1 does not see other SMs' writes).
+__device__ __forceinline__ Q4<float> ldcg_q(const Q4<float>* p) {
+    const float4 x = __ldcg(reinterpret_cast<const float4*>(p));
+    Q4<float> q;
+    q.p[0] = x.x; q.p[1] = x.y; q.p[2] = x.z; q.p[3] = x.w;
+    return q;
+}
+
+// Barrier over the grid of a cooperative launch (every CTA is resident): all writes of every CTA
+// before it are visible after it.  Bounded: false (in every thread of the CTA) when the others have
+// not arrived after 2^23 polls (seconds: far longer than any stage takes, with room for other
+// kernels that hold some of the SMs when the grid is launched).
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target) {
+    __syncthreads();
+    int bad = 0;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        int polls = 0;
+        for (;;) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if (++polls > (1 << 23)) { bad = 1; break; }
+        }
+    }
+    return !__syncthreads_or(bad);
+}
+
+template <int MINB>
+__global__ void __launch_bounds__(kTileCore, MINB) k_titer(TArgs a, TIter it) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    uint32_t* srec = reinterpret_cast<uint32_t*>(sm);
+    uint16_t* scsr = reinterpret_cast<uint16_t*>(sm + it.o_csr);
+    int* shalo = reinterpret_cast<int*>(sm + it.o_halo);
+    Q4<float>* cq = reinterpret_cast<Q4<float>*>(sm + it.o_cq);
+    Q4<float>* cg = reinterpret_cast<Q4<float>*>(sm + it.o_cg);
+    float4* w_t = reinterpret_cast<float4*>(sm + it.o_t);
+    float* w_sp = reinterpret_cast<float*>(sm + it.o_sp);
+    Q4<float>* sqp = reinterpret_cast<Q4<float>*>(sm + it.o_qp);      // previous stage's states
+    float4* slsq = reinterpret_cast<float4*>(sm + it.o_lsq);          // LSQ moments
+    __shared__ __align__(16) TileDesc td;
+    __shared__ __align__(16) TParams tp;
+    __shared__ __align__(8) unsigned long long mbar;
+    __shared__ float redw[4][kTileCore / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t mb = smem_u32(&mbar);
+    const int t = blockIdx.x;
+    if (tid == 0) {
+        td = a.tiles[t];
+        mbar_init(mb, 1);
+    }
+    __syncthreads();
+    // an empty slot (a removed solve's) or a descriptor outside the plan only takes part in the barriers
+    const TileDesc& d = td;
+    const bool live = d.ncore > 0 && d.ncore <= kTileCore && d.n1 >= 0 && d.n2 >= 0 && d.ncore + d.n1 <= it.max_grad &&
+                      d.ncore + d.n1 + d.n2 <= it.max_cells && d.nrc <= it.max_flux && d.nint >= 0 && d.nint <= d.nrc &&
+                      d.nrc <= d.ngeo && d.ngeo <= d.nr && d.nrp >= d.nr && d.ngp >= d.ngeo &&
+                      5 * d.nrp + 3 * d.ngp <= it.max_rec && d.ncsr <= it.max_csr && d.noff <= d.ncsr &&
+                      d.n1 + d.n2 <= d.nhalo && d.nhalo <= it.max_halo && (d.nrp & 3) == 0 && (d.ngp & 3) == 0 &&
+                      (d.ncsr & 7) == 0 && (d.nhalo & 3) == 0 && (d.rec & 3) == 0 && (d.csr & 7) == 0 && (d.halo & 3) == 0;
+    if (!live && d.ncore != 0 && tid == 0) atomicOr(a.err, 4);
+    if (live) {
+        if (tid == 0) {
+            tp = a.P[d.sid];
+            const uint32_t brec = 4u * (uint32_t)(5 * d.nrp + 3 * d.ngp), bcsr = 2u * (uint32_t)d.ncsr,
+                           bhal = 4u * (uint32_t)d.nhalo;
+            mbar_expect_tx(mb, brec + bcsr + bhal);
+            tma_load(srec, a.rec + d.rec, brec, mb);
+            tma_load(scsr, a.csr + d.csr, bcsr, mb);
+            if (bhal) tma_load(shalo, a.halo + d.halo, bhal, mb);
+        }
+        const bool ok = mbar_wait(mb, 0);
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) atomicOr(a.err, 2);
+            return;
+        }
+    }
+    const int ncore = live ? d.ncore : 0, n1 = live ? d.n1 : 0, nh = live ? n1 + d.n2 : 0;
+    const int cbase = d.cbase, c0 = d.c0, nrp = d.nrp, ngp = d.ngp, nrc = live ? d.nrc : 0, nint = d.nint, sid = d.sid;
+    const Consts<float>& k = tp.k;
+    const bool order2 = live && tp.order2 != 0, visc = order2 && tp.ns != 0, squeeze = tp.squeeze != 0;
+    const TileView tv{srec, reinterpret_cast<const float4*>(srec + nrp), reinterpret_cast<const float*>(srec + 5 * nrp),
+                      reinterpret_cast<const float*>(srec + 5 * nrp + ngp),
+                      reinterpret_cast<const float*>(srec + 5 * nrp + 2 * ngp), scsr,
+                      reinterpret_cast<const uint32_t*>(scsr + d.noff), cq, cg};
+    // the core cells' RK data
+    const int gid = c0 + tid;
+    Q4<float> qn, lo, dinc;
+    float dtc = 0.f, sc = 0.f, vc = 1.f, yv = 1.f;
+#pragma unroll
+    for (int j = 0; j < 4; j++) { qn.p[j] = 0.f; lo.p[j] = 0.f; dinc.p[j] = 0.f; }
+    if (tid < ncore) {
+        qn = a.Q[0][gid];
+        cq[tid] = qn;
+        lo = a.Qlo[gid];
+        sc = a.S[gid];
+        vc = a.vol[gid];
+        yv = a.rvol[gid];
+    }
+    if (order2)
+        for (int gI = tid; gI < ncore + n1; gI += blockDim.x) {
+            const int g = gI < ncore ? c0 + gI : cbase + shalo[gI - ncore];
+            slsq[gI] = a.lsq[g];
+            if (squeeze) {
+                sqp[gI] = a.Q[2][g];
+                cg[2 * gI] = a.G[2][2 * (size_t)g];
+                cg[2 * gI + 1] = a.G[2][2 * (size_t)g + 1];
+            }
+        }
+    unsigned target = it.bar0;
+    for (int i = 0; i < it.iterations; i++) {
+        const bool final = i == it.iterations - 1;
+#pragma unroll 1
+        for (int s = 0; s < 3; s++) {
+            const Q4<float>* Qin = s == 0 ? a.Q[0] : s == 1 ? a.Q[1] : a.Q[2];
+            const bool begin = i == 0 && s == 0;      // the previous stage ran in an earlier launch
+            const bool fresh = begin && tp.fresh != 0, init_prims = begin && tp.init_prims != 0;
+            // ---- gather: the ring cells' states (ring 2 only for gradients)
+            for (int h = tid; h < (order2 ? nh : n1); h += blockDim.x) cq[ncore + h] = ldcg_q(Qin + cbase + shalo[h]);
+            const float smax = s == 0 && live && tp.global_dt ? __ldcg(a.smax + sid) : 0.f;
+            __syncthreads();
+            // ---- gradients
+            if (order2) {
+                Q4<float>* Gout = s == 0 ? a.G[0] : s == 1 ? a.G[1] : a.G[2];
+                const bool lim_prev = squeeze && !fresh;
+                for (int gI = tid; gI < ncore + n1; gI += blockDim.x) {
+                    Q4<float> gpx, gpy, gx, gy;
+                    if (lim_prev) { gpx = cg[2 * gI]; gpy = cg[2 * gI + 1]; }
+                    tile_gradient(tv, k, gI, squeeze, lim_prev, init_prims, s == 0, slsq[gI], gpx, gpy,
+                                  [&](int r) { return ldcg_q(Qin + cbase + a.qcell[td.rbase + r]); }, [&] { return sqp[gI]; }, gx, gy);
+                    cg[2 * gI] = gx;
+                    cg[2 * gI + 1] = gy;
+                    sqp[gI] = cq[gI];
+                    if (final && gI < ncore) { Gout[2 * (size_t)(c0 + gI)] = gx; Gout[2 * (size_t)(c0 + gI) + 1] = gy; }
+                }
+                __syncthreads();
+            }
+            // ---- fluxes
+            for (int r = tid; r < nrc; r += blockDim.x) {
+                if (r < nint) tile_flux<true>(tv, k, r, order2, visc, init_prims, s == 2, w_t, w_sp);
+                else tile_flux<false>(tv, k, r, order2, visc, init_prims, s == 2, w_t, w_sp);
+            }
+            __syncthreads();
+            // ---- update
+            float snext = 0.f;
+            float r2[4] = {0.f, 0.f, 0.f, 0.f};
+            if (tid < ncore) {
+                float r4[4];
+                tile_residual(tv, tid, w_t, w_sp, s == 2, yv, r4, snext);
+                if (final && a.R && s == 2) { Q4<float> rr; for (int j = 0; j < 4; j++) rr.p[j] = r4[j]; a.R[gid] = rr; }
+                if (s == 0) {
+                    dtc = fm(k.two_cfl, vc) / (tp.global_dt ? smax : sc);
+                    if (final) a.dt[gid] = dtc;
+                }
+                Q4<float> out, dn = dinc;
+                stage_combine(s, dtc, r4, qn, dinc, lo, dn, out);
+                dinc = dn;
+                (s == 0 ? a.Q[1] : s == 1 ? a.Q[2] : a.Q[0])[gid] = out;
+                cq[tid] = out;
+                if (s == 2) {
+                    qn = out;
+                    sc = snext;
+                    if (final) { a.Qlo[gid] = lo; a.S[gid] = sc; }
+#pragma unroll
+                    for (int j = 0; j < 4; j++) r2[j] = r4[j] * r4[j];
+                }
+                if (!positive(out.p[0]) || !positive(out.p[3])) atomicOr(a.flags + sid, 1);
+            }
+            if (s == 1 && tid == 0 && live && c0 == cbase) {
+                // the solve's first tile: its GLOBAL-dt maximum (read in the first stage, accumulated in
+                // the last) starts again; its history flags (read before the first barrier) end
+                a.smax[sid] = 0.f;
+                if (i == 0) { a.P[sid].fresh = 0; a.P[sid].init_prims = 0; }
+            }
+            if (s == 2 && live) {
+                float m = snext;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) m = max2(m, __shfl_xor_sync(0xffffffffu, m, o));
+                if (lane == 0 && 32 * warp < ncore) atomic_max_pos(a.smax + sid, m);
+                if (a.tpart && final) {   // as the stage kernel: FP32 per warp, FP64 over the warps in order
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) r2[j] += __shfl_xor_sync(0xffffffffu, r2[j], o);
+                    if (lane == 0)
+#pragma unroll
+                        for (int j = 0; j < 4; j++) redw[j][warp] = r2[j];
+                    __syncthreads();
+                    if (tid < 4) {
+                        double sum = 0.0;
+                        for (int w = 0; w < kTileCore / 32; w++) sum += (double)redw[tid][w];
+                        a.tpart[4 * (size_t)t + tid] = sum;
+                    }
+                }
+            }
+            if (final && s == 2) break;
+            target += gridDim.x;
+            if (!grid_barrier(it.bar, target)) {
+                if (tid == 0) atomicOr(a.err, 8);
+                return;
+            }
+        }
     }
 }
 

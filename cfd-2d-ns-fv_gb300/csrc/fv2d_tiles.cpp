@@ -239,7 +239,7 @@ bool check_tile_layout(const TileLayout& T, const DeviceLayout& L, std::string& 
     return true;
 }
 
-bool build_tile_layout(const HostMesh& m, const DeviceLayout& L, TileLayout& T, std::string& err) {
+bool build_tile_layout(const HostMesh& m, const DeviceLayout& L, TileLayout& T, std::string& err, int core) {
     T = TileLayout();
     const int nc = L.nc, nf = L.nf;
     T.nc = nc;
@@ -247,10 +247,10 @@ bool build_tile_layout(const HostMesh& m, const DeviceLayout& L, TileLayout& T, 
     Marks mk(nc, nf);
     int stamp = 0;
     Tile t;
-    // tiles are the renumbering's 256-cell Hilbert blocks; a block that exceeds a capacity (cells
+    // tiles are the renumbering's Hilbert blocks of `core` cells; a block that exceeds a capacity (cells
     // with very many faces) is split in halves until it fits
     std::vector<std::pair<int, int>> todo;
-    for (int c0 = nc - (nc - 1) % kTileCore - 1; c0 >= 0; c0 -= kTileCore) todo.push_back({c0, std::min(kTileCore, nc - c0)});
+    for (int c0 = nc - (nc - 1) % core - 1; c0 >= 0; c0 -= core) todo.push_back({c0, std::min(core, nc - c0)});
     long long recs = 0, r1 = 0, r2 = 0;
     while (!todo.empty()) {
         const auto [c0, n] = todo.back();
@@ -271,6 +271,14 @@ bool build_tile_layout(const HostMesh& m, const DeviceLayout& L, TileLayout& T, 
         todo.push_back({c0, h});
     }
     if (!check_tile_layout(T, L, err)) return false;
+    for (const TileRec& r : T.tiles) {
+        T.max_rec = std::max(T.max_rec, 5 * r.nrp + 3 * r.ngp);
+        T.max_csr = std::max(T.max_csr, r.ncsr);
+        T.max_halo = std::max(T.max_halo, r.nhalo);
+        T.max_cells = std::max(T.max_cells, r.ncore + r.n1 + r.n2);
+        T.max_grad = std::max(T.max_grad, r.ncore + r.n1);
+        T.max_flux = std::max(T.max_flux, r.nrc);
+    }
     T.rec_per_face = nf ? (double)recs / nf : 0.0;
     T.ring1_per_cell = nc ? (double)r1 / nc : 0.0;
     T.ring2_per_cell = nc ? (double)r2 / nc : 0.0;

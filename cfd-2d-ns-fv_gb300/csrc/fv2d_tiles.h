@@ -76,6 +76,9 @@ static_assert(sizeof(TileDesc) == 112, "TileDesc layout");
 struct TileLayout {
     int nc = 0;                          // cells (device order)
     int nc4 = 0;                         // cells rounded up to 4 (per-cell arrays are this long)
+    // largest tile: words of a record block, u16 words of a csr block, ids of a halo list, cells,
+    // gradient (core and ring-1) cells, records with fluxes
+    int max_rec = 0, max_csr = 0, max_halo = 0, max_cells = 0, max_grad = 0, max_flux = 0;
     std::vector<TileRec> tiles;
     std::vector<uint32_t> rec;           // record blocks
     std::vector<int> qcell;              // per record
@@ -91,9 +94,10 @@ struct TileLayout {
 
 struct HostMesh;
 struct DeviceLayout;
-// Build the tile layout of a mesh (device order from build_layout).  Returns false (with a
-// message) only if a single cell needs more than a tile's capacity.
-bool build_tile_layout(const HostMesh& m, const DeviceLayout& L, TileLayout& T, std::string& err);
+// Build the tile layout of a mesh (device order from build_layout): tiles are runs of `core` cells
+// (<= kTileCore; the renumbering's block, so that they are compact).  Returns false (with a message)
+// only if a single cell needs more than a tile's capacity.
+bool build_tile_layout(const HostMesh& m, const DeviceLayout& L, TileLayout& T, std::string& err, int core = kTileCore);
 // Every index the stage kernels derive from the layout stays inside its array or shared-memory
 // region (run by build_tile_layout before a layout is used).
 bool check_tile_layout(const TileLayout& T, const DeviceLayout& L, std::string& err);
