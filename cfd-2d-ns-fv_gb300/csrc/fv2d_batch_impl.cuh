@@ -91,6 +91,7 @@ kb_gradient(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevM
             const Q4<T>* __restrict__ Gprev, Q4<T>* __restrict__ Gout) {
     __shared__ SolveParams<T> sp;
     __shared__ Tile st;
+    const Fp fp;
     const int nt = *ntiles;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         if (threadIdx.x == 0) { st = tiles[t]; sp = P[st.sid]; }
@@ -98,11 +99,11 @@ kb_gradient(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevM
         if (sp.order2) {
             if (sp.squeeze) {
                 for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                    gradient_cell<T, true, sizeof(T) == 8, FV2D_KB_MAXT / 32>(st.start + e, m, Qin, Qprev, Gprev, Gout, sp.k,
+                    gradient_cell<true, true, FV2D_KB_MAXT / 32>(st.start + e, fp, m, Qin, Qprev, Gprev, Gout, sp.k,
                                                                              sp.fresh, sp.init_prims);
             } else {
                 for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                    gradient_cell<T, false>(st.start + e, m, Qin, Qprev, Gprev, Gout, sp.k, sp.fresh, sp.init_prims);
+                    gradient_cell<false>(st.start + e, fp, m, Qin, Qprev, Gprev, Gout, sp.k, sp.fresh, sp.init_prims);
             }
         }
         __syncthreads();
@@ -119,19 +120,20 @@ kb_face(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevMesh<
         Q4<T>* __restrict__ tout, T* __restrict__ sout) {
     __shared__ SolveParams<T> sp;
     __shared__ Tile st;
+    const Fp fp;
     const int nt = *ntiles;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         if (threadIdx.x == 0) { st = tiles[t]; sp = P[st.sid]; }
         __syncthreads();
         if (!sp.order2) {
             for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                face_flux<T, false, false, LAST>(st.start + e, m, Qin, G, tout, sout, sp.k, sp.init_prims);
+                face_flux<false, false, LAST>(st.start + e, fp, m, Qin, G, tout, sout, sp.k, sp.init_prims);
         } else if (sp.ns) {
             for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                face_flux<T, true, true, LAST>(st.start + e, m, Qin, G, tout, sout, sp.k, sp.init_prims);
+                face_flux<true, true, LAST>(st.start + e, fp, m, Qin, G, tout, sout, sp.k, sp.init_prims);
         } else {
             for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                face_flux<T, true, false, LAST>(st.start + e, m, Qin, G, tout, sout, sp.k, sp.init_prims);
+                face_flux<true, false, LAST>(st.start + e, fp, m, Qin, G, tout, sout, sp.k, sp.init_prims);
         }
         __syncthreads();
     }
@@ -147,6 +149,7 @@ kb_update(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevMes
     __shared__ Tile st;
     __shared__ double redd[32];
     __shared__ T redt[32];
+    const Fp fp;
     const int nt = *ntiles;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         if (threadIdx.x == 0) { st = tiles[t]; sp = P[st.sid]; }
@@ -156,8 +159,8 @@ kb_update(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevMes
         double acc[4] = {0, 0, 0, 0};
         for (int e = threadIdx.x; e < st.count; e += blockDim.x) {
             T r[4];
-            const T sn = update_cell<T, STAGE>(st.start + e, m, tface, sface, Qn, Q1, Q2, dt, S, sm, nullptr,
-                                               flags + st.sid, sp.k, sp.global_dt, r, D, Qlo);
+            const T sn = update_cell<STAGE>(st.start + e, fp, m, tface, sface, Qn, Q1, Q2, dt, S, sm, nullptr,
+                                               flags + st.sid, sp.k, sp.global_dt, r);
             if (STAGE == 2) {
                 mx = max2(mx, sn);
 #pragma unroll

@@ -1,4 +1,5 @@
-// Device kernels of the fv2d residual-and-update step, templated on the state precision T.
+// Device kernels of the fv2d residual-and-update step, FP64 engine (and the state transfers and small
+// helpers both precisions share, templated on the state type T).
 //
 // One RK stage = three launches:
 //   k_gradient  (one thread per cell)  LSQ gradient over the cell's faces + squeeze limiter
@@ -8,8 +9,8 @@
 //                                      id, divides by the volume, applies the SSP-RK3 stage, and
 //                                      (last stage) the spectral sums for the next time step
 // Every per-cell sum visits the cell's faces in ascending ORIGINAL face id, the order in which
-// the reference's face loops scatter into the cell, so with T = double and FMA contraction off
-// (-fmad=false) the results are bit-identical to the reference; no atomics touch the state.
+// the reference's face loops scatter into the cell, so with FMA contraction off (-fmad=false) the
+// results are bit-identical to the reference; no atomics touch the state.
 #pragma once
 
 #include <cstdint>
@@ -137,6 +138,58 @@ __device__ __forceinline__ double div3<double>(double a) {
     return __fma_rn(__fma_rn(-3.0, q0, a), y, q0);
 }
 
+// FP64 arithmetic as fused multiply-adds of vector registers.  GB300's FP64 pipe takes a warp's DFMA
+// with three vector-register operands every 16 cycles per SM, but a DADD, a DMUL, or a DFMA with a
+// constant, immediate or uniform-register operand only every 19 (measured with 1,000 operations per
+// thread, 4 to 32 warps on an SM).  So sums and products go as a*1 + b and a*b + (-0), which round
+// exactly as a + b and a*b do, signed zeros included: a*1 is exact, and adding -0 changes no value and
+// no zero's sign.  The constants have to come from memory: from literals or kernel parameters the
+// compiler rebuilds the slower forms.
+// Together with the exact scalings of face_flux, on the 1M-cell NS cylinder: face kernel 2.19 -> 1.75 ms
+// (FP64 pipe busy 94.5 % of the time), gradient 0.40 -> 0.38, update 0.135 -> 0.115; 8.37 -> 6.87 ms per
+// iteration.
+// half: a factor of 1/2 enters through the multiply-add that uses it (x - m/2 = fma(m, -1/2, x), as
+// m/2 is exact), so it costs no operation of its own.
+__device__ double g_fp64_consts[4] = {1.0, -0.0, 0.5, 0.25};
+struct Fp {
+    double one, nz, half;
+    __device__ __forceinline__ Fp() {
+        one = g_fp64_consts[0];
+        nz = g_fp64_consts[1];
+        half = g_fp64_consts[2];
+    }
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(a, one, -b); }
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nz); }
+};
+
+// Several quotients by one denominator b: y = RN(1/b) and yl the digits of 1/b after it, so that
+// q0 = RN(a*y + RN(a*yl)) is a/b within 2^-50 ulp before its rounding, hence faithful; then the residual
+// a - b*q0 is exact and q0 + (a - b*q0)*y rounds to the correctly rounded a/b (Markstein, as above:
+// y correctly rounded, q0 faithful).  Four operations a quotient and two per denominator, against
+// five for the two residual corrections of Recip.  Same operand range; a zero numerator gives the exact
+// signed zero.  Tested bit for bit against IEEE division.
+struct Divisor {
+    double b, y, yl;
+    __device__ __forceinline__ Divisor(double b_, double y_, const Fp& f) {
+        b = b_;
+        y = y_;
+        yl = f.mul(__fma_rn(-b_, y_, f.one), y_);
+    }
+    __device__ __forceinline__ Divisor(double b_, const Fp& f) {
+        b = b_;
+        y = __drcp_rn(b_);
+        yl = f.mul(__fma_rn(-b_, y, f.one), y);
+    }
+    __device__ __forceinline__ double div(double a, const Fp& f) const {
+        const double q0 = __fma_rn(a, y, f.mul(a, yl));
+        const double q = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+        const int ha = __double2hiint(a);
+        const bool zero = ((ha << 1) | __double2loint(a)) == 0;
+        return zero ? __hiloint2double((ha ^ __double2hiint(b)) & (int)0x80000000, 0) : q;
+    }
+};
+
 // +0 - x, IEEE round to nearest, for a term (V A) that is identically +0 (V = +0, area A >= +0):
 // -x, and +0 when x is a zero of either sign
 __device__ __forceinline__ double zero_minus(double x) {
@@ -148,15 +201,15 @@ __device__ __forceinline__ float zero_minus(float x) {
     return (b << 1) == 0 ? 0.0f : __int_as_float(b);
 }
 
-// prims() with the reciprocal of rho shared by u, v (and returned for P/rho)
-template <class T>
-__device__ __forceinline__ void prims_r(const T p[4], const Consts<T>& k, T& rho, T& u, T& v, T& P, T& y) {
-    rho = p[0];
-    const T E = p[3];
-    y = Recip<T>::of(rho);
-    u = Recip<T>::div(p[1], rho, y);
-    v = Recip<T>::div(p[2], rho, y);
-    P = (E - (T(0.5) * rho * (u * u + v * v))) * k.gm1;
+// prims() with rho's divisor shared by u, v (and returned for P/rho)
+__device__ __forceinline__ Divisor prims_r(const double p[4], const Consts<double>& k, const Fp& f, double& u, double& v,
+                                           double& P) {
+    const Divisor r(p[0], f);
+    u = r.div(p[1], f);
+    v = r.div(p[2], f);
+    const double m = f.mul(p[0], f.add(f.mul(u, u), f.mul(v, v)));
+    P = f.mul(__fma_rn(m, -f.half, p[3]), k.gm1);   // E - (0.5 rho (u^2 + v^2)), the product's half exact
+    return r;
 }
 
 // class_flow::updateQ (class_flow.hpp:28-34)
@@ -181,9 +234,6 @@ __device__ __forceinline__ T pick4(const T a[4], int j) {
     return j == 0 ? a[0] : j == 1 ? a[1] : j == 2 ? a[2] : a[3];
 }
 
-#ifndef FV2D_FP32_BLOCK
-#define FV2D_FP32_BLOCK 128   // threads per block of the FP32 single-solve gradient and face kernels
-#endif
 #ifndef FV2D_FP64_BLOCK
 #define FV2D_FP64_BLOCK 128   // threads per block of the FP64 gradient and face kernels
 #endif
@@ -200,11 +250,12 @@ struct WarpQ {
     double quo[WARPS][FV2D_WARPQ_CAP];                              // the checks' quotients
 };
 
-template <class T, bool SQUEEZE, bool WARPQ = false, int QWARPS = FV2D_FP64_BLOCK / 32>
-__device__ __forceinline__ void gradient_cell(int c, const DevMesh<T>& m, const Q4<T>* __restrict__ Q,
-                                              const Q4<T>* __restrict__ Qprev, const Q4<T>* __restrict__ Gprev,
-                                              Q4<T>* __restrict__ Gout, const Consts<T>& k, int first_stage,
+template <bool SQUEEZE, bool WARPQ = false, int QWARPS = FV2D_FP64_BLOCK / 32>
+__device__ __forceinline__ void gradient_cell(int c, const Fp& fp, const DevMesh<double>& m, const Q4<double>* __restrict__ Q,
+                                              const Q4<double>* __restrict__ Qprev, const Q4<double>* __restrict__ Gprev,
+                                              Q4<double>* __restrict__ Gout, const Consts<double>& k, int first_stage,
                                               int init_prims) {
+    using T = double;
     const int* __restrict__ inc_off = m.inc_off;
     const int* __restrict__ inc = m.inc;
     const int* __restrict__ nbr = m.nbr;
@@ -236,7 +287,7 @@ __device__ __forceinline__ void gradient_cell(int c, const DevMesh<T>& m, const 
             const T* q2 = side == 0 ? qn.p : qc.p;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                d[j] = q2[j] - q1[j];
+                d[j] = fp.sub(q2[j], q1[j]);
                 if (SQUEEZE) {
                     qmin[j] = min2(qmin[j], min2(q1[j], q2[j]));
                     qmax[j] = max2(qmax[j], max2(q1[j], q2[j]));
@@ -245,12 +296,12 @@ __device__ __forceinline__ void gradient_cell(int c, const DevMesh<T>& m, const 
         } else {
             if (nb == -1) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) d[j] = k.q_inf[j] - qc.p[j];
+                for (int j = 0; j < 4; j++) d[j] = fp.sub(k.q_inf[j], qc.p[j]);
             } else if (nb == -2 || nb == -4) {
-                T rho, u, v, P, yr;
+                T rho, u, v, P;
                 if (init_prims) { rho = k.rho_inf; u = k.u_inf; v = k.v_inf; P = k.P_inf; }
-                else if (nb == -2) prims_r(qc.p, k, rho, u, v, P, yr);
-                else { const Q4<T> qq = ldq(Q, qcell[f]); prims_r(qq.p, k, rho, u, v, P, yr); }
+                else if (nb == -2) { rho = qc.p[0]; prims_r(qc.p, k, fp, u, v, P); }
+                else { const Q4<T> qq = ldq(Q, qcell[f]); rho = qq.p[0]; prims_r(qq.p, k, fp, u, v, P); }
                 T gq[4];
                 if (nb == -2) {        // slip wall: reflect the cell velocity (cell_gradient.cpp:43-55)
                     const T fnx = g.nx[f], fny = g.ny[f];
@@ -260,7 +311,7 @@ __device__ __forceinline__ void gradient_cell(int c, const DevMesh<T>& m, const 
                     cons(rho, -u, -v, P, k, gq);
                 }
 #pragma unroll
-                for (int j = 0; j < 4; j++) d[j] = gq[j] - qc.p[j];
+                for (int j = 0; j < 4; j++) d[j] = fp.sub(gq[j], qc.p[j]);
             } else {
 #pragma unroll
                 for (int j = 0; j < 4; j++) d[j] = T(0);
@@ -271,22 +322,22 @@ __device__ __forceinline__ void gradient_cell(int c, const DevMesh<T>& m, const 
         }
         const T fx = ig.p[0], fy = ig.p[1];
 #pragma unroll
-        for (int j = 0; j < 4; j++) { sx[j] += d[j] * fx; sy[j] += d[j] * fy; }
+        for (int j = 0; j < 4; j++) { sx[j] = fp.add(sx[j], fp.mul(d[j], fx)); sy[j] = fp.add(sy[j], fp.mul(d[j], fy)); }
     }
     const T ixx = (T)m.Ixx[c], iyy = (T)m.Iyy[c], ixy = (T)m.Ixy[c];
     Q4<T> gx, gy;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        gx.p[j] = (sx[j] * iyy - sy[j] * ixy);
-        gy.p[j] = (sy[j] * ixx - sx[j] * ixy);
+        gx.p[j] = fp.sub(fp.mul(sx[j], iyy), fp.mul(sy[j], ixy));
+        gy.p[j] = fp.sub(fp.mul(sy[j], ixx), fp.mul(sx[j], ixy));
     }
     if (SQUEEZE) {
         T phi[4] = {T(1), T(1), T(1), T(1)};
         Q4<T> qp, gpx, gpy;
-        const Q4<T>* __restrict__ fval = sizeof(T) == 8 ? m.fval : nullptr;   // FP64 engine only
+        const Q4<T>* __restrict__ fval = m.fval;
         if (!first_stage && !fval) { qp = ldq(Qprev, c); gpx = ldq(Gprev, 2 * c); gpy = ldq(Gprev, 2 * c + 1); }
-        if constexpr (sizeof(T) == 8) {
-            // FP64: only a minority of the (incidence, component) checks bound the face value and
+        {
+            // Only a minority of the (incidence, component) checks bound the face value and
             // need a quotient, but a conditional IEEE division is if-converted (computed for every
             // check).  So one pass flags the checks that need one (bit 4*(incidence - i0) + component,
             // 16 incidences per word) and a second loop takes one flagged check per trip - one
@@ -409,50 +460,31 @@ __device__ __forceinline__ void gradient_cell(int c, const DevMesh<T>& m, const 
                     for (int jj = 0; jj < 4; jj++) phi[jj] = jj == j ? ph : phi[jj];
                 }
             }
-        } else {
-            for (int i = b; i < e; i++) {
-                const Q4<T> ig = ldq(m.igeo, i);
-                const T dx = ig.p[2], dy = ig.p[3];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const T qf = first_stage ? T(-101) : qp.p[j] + gpx.p[j] * dx + gpy.p[j] * dy;
-                    T ph = T(1);
-                    if (less(qf, qmin[j])) ph = (qmin[j] - qc.p[j]) / (qf - qc.p[j]);
-                    else if (less(qmax[j], qf)) ph = (qmax[j] - qc.p[j]) / (qf - qc.p[j]);
-                    phi[j] = min2(ph, phi[j]);
-                }
-            }
         }
 #pragma unroll
-        for (int j = 0; j < 4; j++) { gx.p[j] = gx.p[j] * phi[j]; gy.p[j] = gy.p[j] * phi[j]; }
+        for (int j = 0; j < 4; j++) { gx.p[j] = fp.mul(gx.p[j], phi[j]); gy.p[j] = fp.mul(gy.p[j], phi[j]); }
     }
     Gout[2 * c] = gx;
     Gout[2 * c + 1] = gy;
 }
 
-// Occupancy: the FP32 kernels are latency-bound gathers, so their register use is capped for more
-// resident warps.  The FP64 kernels are FP64-pipe-bound; their block size and minimum resident
-// blocks (register cap) set how many warps cover the pipe's latency.
+// Occupancy: the kernels are FP64-pipe-bound; their block size and minimum resident blocks (register
+// cap) set how many warps cover the pipe's latency.
 #ifndef FV2D_FP64_GMINB
 #define FV2D_FP64_GMINB 8   // 8 x 128 threads at 64 registers (spilling), 8 x 23 KB of shared memory:
                             // 4 % faster than half the warps at 128 registers
 #endif
 #ifndef FV2D_FP64_FMINB
-#define FV2D_FP64_FMINB 4   // 4 x 128 threads at 116 registers
+#define FV2D_FP64_FMINB 4   // 4 x 128 threads at up to 128 registers
 #endif
-template <class T>
-constexpr int kStageBlock = sizeof(T) == 4 ? FV2D_FP32_BLOCK : FV2D_FP64_BLOCK;   // gradient and face kernels
-
-#ifndef FV2D_KG_MINB32
-#define FV2D_KG_MINB32 8   // 8 x 128 threads at 61 registers, no spills: 3.5 % faster than 10 at 48
-#endif
-template <class T, bool SQUEEZE>
-__global__ void __launch_bounds__(kStageBlock<T>, sizeof(T) == 4 ? FV2D_KG_MINB32 : FV2D_FP64_GMINB)
-k_gradient(int nc, DevMesh<T> m, const Q4<T>* __restrict__ Q, const Q4<T>* __restrict__ Qprev,
-           const Q4<T>* __restrict__ Gprev, Q4<T>* __restrict__ Gout, Consts<T> k, int first_stage, int init_prims) {
+template <bool SQUEEZE>
+__global__ void __launch_bounds__(FV2D_FP64_BLOCK, FV2D_FP64_GMINB)
+k_gradient(int nc, DevMesh<double> m, const Q4<double>* __restrict__ Q, const Q4<double>* __restrict__ Qprev,
+           const Q4<double>* __restrict__ Gprev, Q4<double>* __restrict__ Gout, Consts<double> k, int first_stage, int init_prims) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc) return;
-    gradient_cell<T, SQUEEZE, sizeof(T) == 8>(c, m, Q, Qprev, Gprev, Gout, k, first_stage, init_prims);
+    const Fp fp;
+    gradient_cell<SQUEEZE, true>(c, fp, m, Q, Qprev, Gprev, Gout, k, first_stage, init_prims);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -461,166 +493,187 @@ k_gradient(int nc, DevMesh<T> m, const Q4<T>* __restrict__ Q, const Q4<T>* __res
 // (class_f.hpp:41-50, rusanov.cpp:20-36) and the face's residual contribution (res.cpp:81-89).
 // Writes t = (V*A) - (F*A) per face and, on the last stage of an iteration, the spectral term
 // (|Vn_avg| + c_avg)*A that the next time step sums (ssp_rk3.cpp:28-36).
-template <class T, bool ORDER2, bool NS, bool LAST>
-__device__ __forceinline__ void face_flux(int f, const DevMesh<T>& m, const Q4<T>* __restrict__ Q,
-                                          const Q4<T>* __restrict__ G, Q4<T>* __restrict__ tout,
-                                          T* __restrict__ sout, const Consts<T>& k, int init_prims) {
-    const FaceGeo<T>& g = m.g;
+// Powers of two travel through the formulas as exact scalings instead of operations: the average
+// state's sums S = L + R stand for 2 (L + R)/2, the wave speed t = |vn1 + vn2| + (c1 + c2) for 4 lambda,
+// the flux F2 for 2 F against half the area, the viscous flux V2 for 2 V (mu and k enter doubled), and
+// the remaining halves ride on multiply-adds.  Every rounded intermediate is the reference's times a
+// power of two, so the results are the same bits.  338 FP64 operations for an NS interior face.
+template <bool ORDER2, bool NS, bool LAST>
+__device__ __forceinline__ void face_flux(int f, const Fp& fp, const DevMesh<double>& m, const Q4<double>* __restrict__ Q,
+                                          const Q4<double>* __restrict__ G, Q4<double>* __restrict__ tout,
+                                          double* __restrict__ sout, const Consts<double>& k, int init_prims) {
+    const FaceGeo<double>& g = m.g;
     const int c1 = m.fc1[f], c2 = m.fc2[f];
-    const T fnx = g.nx[f], fny = g.ny[f], A = g.area[f];
-    const Q4<T> q1 = ldq(Q, c1);
-    Q4<T> g1x, g1y;
+    const double fnx = g.nx[f], fny = g.ny[f], A = g.area[f];
+    const Q4<double> q1 = ldq(Q, c1);
+    Q4<double> g1x, g1y;
     if (ORDER2) { g1x = ldq(G, 2 * c1); g1y = ldq(G, 2 * c1 + 1); }
-    else {
-#pragma unroll
-        for (int j = 0; j < 4; j++) { g1x.p[j] = T(0); g1y.p[j] = T(0); }
-    }
     // the right cell's loads are issued now, beside the left cell's (a boundary face, c2 < 0,
     // loads cell c1's row instead and never uses it), so the two gathers overlap
     const int c2l = c2 >= 0 ? c2 : c1;
-    const Q4<T> q2l = ldq(Q, c2l);
-    Q4<T> g2xl, g2yl;
-    if (ORDER2) { g2xl = ldq(G, 2 * c2l); g2yl = ldq(G, 2 * c2l + 1); }
-    T L[4], Rq[4];
-    {
-        const T dx = g.c1dx[f], dy = g.c1dy[f];
+    const Q4<double> q2 = ldq(Q, c2l);
+    Q4<double> g2x, g2y;
+    if (ORDER2) { g2x = ldq(G, 2 * c2l); g2y = ldq(G, 2 * c2l + 1); }
+    double L[4], Rq[4];
+    // first order: q + 0 dx + 0 dy is q, but for a -0 that meets a +0 product
+    auto first_order = [&](double q, double dx, double dy) {
+        const bool pos = (__double2hiint(dx) & __double2hiint(dy)) >= 0;
+        return pos && __double_as_longlong(q) == (long long)0x8000000000000000ULL ? 0.0 : q;
+    };
+    if (ORDER2) {
+        const double dx = g.c1dx[f], dy = g.c1dy[f];
 #pragma unroll
-        for (int j = 0; j < 4; j++) L[j] = q1.p[j] + g1x.p[j] * dx + g1y.p[j] * dy;
+        for (int j = 0; j < 4; j++) L[j] = fp.add(fp.add(q1.p[j], fp.mul(g1x.p[j], dx)), fp.mul(g1y.p[j], dy));
+    } else {
+        const double dx = g.c1dx[f], dy = g.c1dy[f];
+#pragma unroll
+        for (int j = 0; j < 4; j++) L[j] = first_order(q1.p[j], dx, dy);
     }
-    T lrho, lu, lv, lP, ly;
-    prims_r(L, k, lrho, lu, lv, lP, ly);
-    const T lc = sqrt(k.gamma * Recip<T>::div(lP, lrho, ly));
-    Q4<T> q2, g2x, g2y;
+    const double lrho = L[0];
+    double lu, lv, lP;
+    const Divisor ld = prims_r(L, k, fp, lu, lv, lP);
+    const double lc = sqrt(k.gamma * ld.div(lP, fp));
     if (c2 >= 0) {
-        q2 = q2l;
-        if (ORDER2) { g2x = g2xl; g2y = g2yl; }
-        else {
+        if (ORDER2) {
+            const double dx = g.c2dx[f], dy = g.c2dy[f];
 #pragma unroll
-            for (int j = 0; j < 4; j++) { g2x.p[j] = T(0); g2y.p[j] = T(0); }
+            for (int j = 0; j < 4; j++) Rq[j] = fp.add(fp.add(q2.p[j], fp.mul(g2x.p[j], dx)), fp.mul(g2y.p[j], dy));
+        } else {
+            const double dx = g.c2dx[f], dy = g.c2dy[f];
+#pragma unroll
+            for (int j = 0; j < 4; j++) Rq[j] = first_order(q2.p[j], dx, dy);
         }
-        const T dx = g.c2dx[f], dy = g.c2dy[f];
-#pragma unroll
-        for (int j = 0; j < 4; j++) Rq[j] = q2.p[j] + g2x.p[j] * dx + g2y.p[j] * dy;
     } else if (c2 == -1) {
 #pragma unroll
         for (int j = 0; j < 4; j++) Rq[j] = k.q_inf[j];
     } else if (c2 == -2) {
-        const T vn = lu * fnx + lv * fny;
-        cons(lrho, lu - T(2.0) * vn * fnx, lv - T(2.0) * vn * fny, lP, k, Rq);
+        const double vn = lu * fnx + lv * fny;
+        cons(lrho, lu - 2.0 * vn * fnx, lv - 2.0 * vn * fny, lP, k, Rq);
     } else if (c2 == -3) {
 #pragma unroll
         for (int j = 0; j < 4; j++) Rq[j] = L[j];
     } else {
         cons(lrho, -lu, -lv, lP, k, Rq);
     }
-    if constexpr (sizeof(T) == 8) {
-        if (m.fval) {   // the next squeeze's stale face values (BC faces: the c1 side only)
-            Q4<T> lq, rq;
+    if (m.fval) {   // the next squeeze's stale face values (BC faces: the c1 side only)
+        Q4<double> lq, rq;
 #pragma unroll
-            for (int j = 0; j < 4; j++) { lq.p[j] = L[j]; rq.p[j] = Rq[j]; }
-            m.fval[2 * f] = lq;
-            if (c2 >= 0) m.fval[2 * f + 1] = rq;
-        }
+        for (int j = 0; j < 4; j++) { lq.p[j] = L[j]; rq.p[j] = Rq[j]; }
+        m.fval[2 * f] = lq;
+        if (c2 >= 0) m.fval[2 * f + 1] = rq;
     }
-    T rrho, ru, rv, rP, ry_;
-    prims_r(Rq, k, rrho, ru, rv, rP, ry_);
-    const T rc = sqrt(k.gamma * Recip<T>::div(rP, rrho, ry_));
+    const double rrho = Rq[0];
+    double ru, rv, rP;
+    const Divisor rd = prims_r(Rq, k, fp, ru, rv, rP);
+    const double rc = sqrt(k.gamma * rd.div(rP, fp));
 
-    // Rusanov
-    const T vn1 = lu * fnx + lv * fny;
-    const T vn2 = ru * fnx + rv * fny;
-    const T F1[4] = {lrho * vn1, lrho * lu * vn1 + lP * fnx, lrho * lv * vn1 + lP * fny, vn1 * (L[3] + lP)};
-    const T F2[4] = {rrho * vn2, rrho * ru * vn2 + rP * fnx, rrho * rv * vn2 + rP * fny, vn2 * (Rq[3] + rP)};
-    const T vna = (vn1 + vn2) / T(2);
-    const T ca = (lc + rc) / T(2);
-    const T lam = (fabs(vna) + ca) / T(2);
-    T Fr[4];
+    // Rusanov: F2 = 2 Fr = (F1 + F2) - (t/2)(R - L), t = 4 lambda = 2 (|Vn_avg| + c_avg)
+    const double vn1 = fp.add(fp.mul(lu, fnx), fp.mul(lv, fny)), vn2 = fp.add(fp.mul(ru, fnx), fp.mul(rv, fny));
+    const double t4 = fp.add(fabs(fp.add(vn1, vn2)), fp.add(lc, rc));
+    const double Ah = fp.mul(A, fp.half);
+    double F2[4];
+    if (k.roe) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) Fr[j] = k.roe ? T(-101) : (F1[j] + F2[j]) / T(2) - lam * (Rq[j] - L[j]);
+        for (int j = 0; j < 4; j++) F2[j] = -202.0;
+    } else {
+        const double X[4] = {
+            fp.add(fp.mul(lrho, vn1), fp.mul(rrho, vn2)),
+            fp.add(fp.add(fp.mul(fp.mul(lrho, lu), vn1), fp.mul(lP, fnx)), fp.add(fp.mul(fp.mul(rrho, ru), vn2), fp.mul(rP, fnx))),
+            fp.add(fp.add(fp.mul(fp.mul(lrho, lv), vn1), fp.mul(lP, fny)), fp.add(fp.mul(fp.mul(rrho, rv), vn2), fp.mul(rP, fny))),
+            fp.add(fp.mul(vn1, fp.add(L[3], lP)), fp.mul(vn2, fp.add(Rq[3], rP)))};
+#pragma unroll
+        for (int j = 0; j < 4; j++) F2[j] = __fma_rn(fp.mul(t4, fp.sub(Rq[j], L[j])), -fp.half, X[j]);
+    }
 
-    // viscous flux (first order never adds it: res.cpp:27-29,50-53)
-    T V[4] = {T(0), T(0), T(0), T(0)};
+    // viscous flux, V2 = 2 V (first order never adds it: res.cpp:27-29,50-53)
+    double V2[4] = {0.0, 0.0, 0.0, 0.0};
     if (NS && ORDER2) {
-        T Aq[4];
+        double S[4];   // twice the average state
 #pragma unroll
-        for (int j = 0; j < 4; j++) Aq[j] = T(0.5) * (L[j] + Rq[j]);
-        T arho, au, av, aP, ya;
-        prims_r(Aq, k, arho, au, av, aP, ya);
-        T ux = T(0), uy = T(0), vx = T(0), vy = T(0), Px = T(0), Py = T(0), rx = T(0), ry = T(0);
+        for (int j = 0; j < 4; j++) S[j] = fp.add(L[j], Rq[j]);
+        const Divisor sd(S[0], fp);
+        const double au = sd.div(S[1], fp), av = sd.div(S[2], fp);
+        const double ke = fp.add(fp.mul(au, au), fp.mul(av, av));
+        const double aP2 = fp.mul(__fma_rn(fp.mul(S[0], ke), -fp.half, S[3]), k.gm1);   // twice the pressure
+        double ux = 0.0, uy = 0.0, vx = 0.0, vy = 0.0, Px = 0.0, Py = 0.0, rx = 0.0, ry = 0.0;
         bool have = true;
         if (c2 >= 0) {
-            const T ad = fabs(g.dist[f]);
-            const T yd = m.rdist[f];   // Recip<T>::of(ad), precomputed
+            const double ad = fabs(g.dist[f]);
+            const Divisor dd(ad, m.rdist[f], fp);   // 1/|dist| precomputed
             // unit tangent p1 -> p2 (readmesh.cpp:400-406) from the normal: mx = dx/|d| = -ny and
             // my = dy/|d| = nx, bit for bit (same |d| expression, sign-symmetric rounding)
-            const T mxf = -fny, myf = fnx, lxf = g.lx[f], lyf = g.ly[f];
-            T dQx[4], dQy[4];
+            const double mxf = -fny, myf = fnx, lxf = g.lx[f], lyf = g.ly[f];
+            double dQx[4], dQy[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const T dl = Recip<T>::div(q2.p[j] - q1.p[j], ad, yd);
-                const T dm = T(0.5) * (g1x.p[j] * mxf + g1y.p[j] * myf + g2x.p[j] * mxf + g2y.p[j] * myf);
-                dQy[j] = dl * lyf + dm * lyf;
-                dQx[j] = dl * lxf + dm * lxf;
+                const double dl = dd.div(fp.sub(q2.p[j], q1.p[j]), fp);
+                const double dm2 = fp.add(fp.add(fp.add(fp.mul(g1x.p[j], mxf), fp.mul(g1y.p[j], myf)), fp.mul(g2x.p[j], mxf)),
+                                          fp.mul(g2y.p[j], myf));   // twice the tangential derivative
+                dQy[j] = __fma_rn(fp.mul(dm2, lyf), fp.half, fp.mul(dl, lyf));
+                dQx[j] = __fma_rn(fp.mul(dm2, lxf), fp.half, fp.mul(dl, lxf));
             }
+            // quotients by S0 = 2 rho are half of those by rho
             rx = dQx[0];
-            ux = dQx[1] - Recip<T>::div(rx * au, arho, ya);
-            vx = dQx[2] - Recip<T>::div(rx * av, arho, ya);
+            ux = __fma_rn(sd.div(fp.mul(rx, au), fp), -2.0, dQx[1]);
+            vx = __fma_rn(sd.div(fp.mul(rx, av), fp), -2.0, dQx[2]);
             ry = dQy[0];
-            uy = dQy[1] - Recip<T>::div(ry * au, arho, ya);
-            vy = dQy[2] - Recip<T>::div(ry * au, arho, ya);   // reconstruction.cpp:155 uses u
-            Px = k.gm1 * (dQx[3] - T(0.5) * rx * (au * au + av * av) - arho * (au * ux + av * vx));
-            Py = k.gm1 * (dQy[3] - T(0.5) * ry * (au * au + av * av) - arho * (au * uy + av * vy));
+            const double ryu = sd.div(fp.mul(ry, au), fp);
+            uy = __fma_rn(ryu, -2.0, dQy[1]);
+            vy = __fma_rn(ryu, -2.0, dQy[2]);   // reconstruction.cpp:155 uses u
+            Px = fp.mul(k.gm1, __fma_rn(fp.mul(S[0], fp.add(fp.mul(au, ux), fp.mul(av, vx))), -fp.half,
+                                        __fma_rn(fp.mul(rx, ke), -fp.half, dQx[3])));
+            Py = fp.mul(k.gm1, __fma_rn(fp.mul(S[0], fp.add(fp.mul(au, uy), fp.mul(av, vy))), -fp.half,
+                                        __fma_rn(fp.mul(ry, ke), -fp.half, dQy[3])));
         } else if (c2 == -4) {
-            const T d1x = g.c1dx[f], d1y = g.c1dy[f];
-            const T dn = fabs(sqrt(d1x * d1x + d1y * d1y));
-            T cu, cv;
+            const double d1x = g.c1dx[f], d1y = g.c1dy[f];
+            const double dn = fabs(sqrt(d1x * d1x + d1y * d1y));
+            double cu, cv;
             if (init_prims) { cu = k.u_inf; cv = k.v_inf; }
             else { cu = q1.p[1] / q1.p[0]; cv = q1.p[2] / q1.p[0]; }
-            const T ydn = Recip<T>::of(dn);
-            const T dudn = Recip<T>::div(-cu, dn, ydn), dvdn = Recip<T>::div(-cv, dn, ydn);
+            const Divisor nd(dn, fp);
+            const double dudn = nd.div(-cu, fp), dvdn = nd.div(-cv, fp);
             ux = dudn * fnx; uy = dudn * fny;
             vx = dvdn * fnx; vy = dvdn * fny;
         } else if (c2 == -2) {
             have = false;   // SLIP_WALL with NS: tau and grad T keep their initial zeros (:104-106)
         }
-        T txx, txy, tyy, dTx, dTy;
+        double txx, txy, tyy, dTx, dTy;   // twice the stresses; half the temperature derivatives
         if (have) {
-            const T third = div3(ux + vy);
-            txx = T(2) * k.mu * (ux - third);
-            txy = k.mu * (uy + vx);
-            tyy = T(2) * k.mu * (vy - third);
-            const T den = k.R * arho * arho, yden = Recip<T>::of(den);
-            dTx = Recip<T>::div(Px * arho - rx * aP, den, yden);
-            dTy = Recip<T>::div(Py * arho - ry * aP, den, yden);
+            const double third = div3(fp.add(ux, vy)), mu2 = 2.0 * k.mu, mu4 = 4.0 * k.mu;
+            txx = fp.mul(mu4, fp.sub(ux, third));
+            txy = fp.mul(mu2, fp.add(uy, vx));
+            tyy = fp.mul(mu4, fp.sub(vy, third));
+            const double den = fp.mul(fp.mul(k.R, S[0]), S[0]), yden = __drcp_rn(den);   // 4 R rho^2
+            dTx = Recip<double>::div(fp.sub(fp.mul(Px, S[0]), fp.mul(rx, aP2)), den, yden);
+            dTy = Recip<double>::div(fp.sub(fp.mul(Py, S[0]), fp.mul(ry, aP2)), den, yden);
         } else {
-            txx = T(0); txy = T(0); tyy = T(0); dTx = T(0); dTy = T(0);
+            txx = 0.0; txy = 0.0; tyy = 0.0; dTx = 0.0; dTy = 0.0;
         }
-        V[0] = T(0);
-        V[1] = txx * fnx + txy * fny;
-        V[2] = txy * fnx + tyy * fny;
-        V[3] = fnx * (au * txx + av * txy + k.k * dTx) + fny * (au * txy + av * tyy + k.k * dTy);
+        const double k4 = 4.0 * k.k;
+        V2[1] = fp.add(fp.mul(txx, fnx), fp.mul(txy, fny));
+        V2[2] = fp.add(fp.mul(txy, fnx), fp.mul(tyy, fny));
+        V2[3] = fp.add(fp.mul(fnx, fp.add(fp.add(fp.mul(au, txx), fp.mul(av, txy)), fp.mul(k4, dTx))),
+                       fp.mul(fny, fp.add(fp.add(fp.mul(au, txy), fp.mul(av, tyy)), fp.mul(k4, dTy))));
     }
-    Q4<T> t;
+    Q4<double> t;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         // (V*A) - (F*A); V[0] is always +0, and all of V is +0 for Euler and first order
-        if (j == 0 || !(NS && ORDER2)) t.p[j] = zero_minus(Fr[j] * A);
-        else t.p[j] = (V[j] * A) - (Fr[j] * A);
+        if (j == 0 || !(NS && ORDER2)) t.p[j] = zero_minus(fp.mul(F2[j], Ah));
+        else t.p[j] = fp.sub(fp.mul(V2[j], Ah), fp.mul(F2[j], Ah));
     }
     tout[f] = t;
-    if (LAST) sout[f] = k.roe ? (fabs(k.vn0) + k.c0) * A : (fabs(vna) + ca) * A;
+    if (LAST) sout[f] = k.roe ? (fabs(k.vn0) + k.c0) * A : fp.mul(t4, Ah);
 }
 
-#ifndef FV2D_KF_MINB32
-#define FV2D_KF_MINB32 10   // 10 x 128 threads at 48 registers (16 B spill): 11 % faster than 8 at 63
-#endif
-template <class T, bool ORDER2, bool NS, bool LAST>
-__global__ void __launch_bounds__(kStageBlock<T>, sizeof(T) == 4 ? FV2D_KF_MINB32 : FV2D_FP64_FMINB)
-k_face(int nf, DevMesh<T> m, const Q4<T>* __restrict__ Q, const Q4<T>* __restrict__ G, Q4<T>* __restrict__ tout,
-       T* __restrict__ sout, Consts<T> k, int init_prims) {
+template <bool ORDER2, bool NS, bool LAST>
+__global__ void __launch_bounds__(FV2D_FP64_BLOCK, FV2D_FP64_FMINB)
+k_face(int nf, DevMesh<double> m, const Q4<double>* __restrict__ Q, const Q4<double>* __restrict__ G, Q4<double>* __restrict__ tout,
+       double* __restrict__ sout, Consts<double> k, int init_prims) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nf) return;
-    face_flux<T, ORDER2, NS, LAST>(f, m, Q, G, tout, sout, k, init_prims);
+    const Fp fp;
+    face_flux<ORDER2, NS, LAST>(f, fp, m, Q, G, tout, sout, k, init_prims);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -673,37 +726,27 @@ k_spectral_init(int nc, const int* __restrict__ inc_off, const int* __restrict__
 // STAGE 1: Q2 = 0.75*Qn + 0.25*Q1 + 0.25*dt*R
 // STAGE 2: Qn = 1/3*Qn + 2/3*Q2 + 2/3*dt*R, and the spectral sums for the next iteration.
 // Non-physical results (rho <= 0, E <= 0, NaN) raise bit 0 of *flag; values are kept as computed.
-// FP32 keeps the RK increments in delta form and the base state as a compensated pair
-// (hi + lo, error-free TwoSum), so increments below half an ulp of the state are not lost:
-//   D1 = dt R1,               Q1 = hi + D1
-//   D2 = D1/4 + dt R2 / 4,    Q2 = hi + D2
-//   (hi, lo) += 2/3 D2 + 2/3 dt R3
-// which is the SSP-RK3 combination of ssp_rk3.cpp:50-77 rewritten about Qn.  Gradients and fluxes
-// read the FP32 stage states (hi, Q1, Q2).  FP64 (D == nullptr) keeps the reference's expressions.
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     s = a + b;
     const float bp = s - a;
     e = (a - (s - bp)) + (b - bp);
 }
 
-// Incidences whose loads the residual gather issues together: 4 for FP64 (4.6 % faster k_update);
-// 1 for FP32, where the wider chunk's registers cost the batch kernel more than it gains.
-template <class T>
-constexpr int kUpdChunk = sizeof(T) == 8 ? 4 : 1;
+constexpr int kUpdChunk = 4;   // incidences whose loads the residual gather issues together (4.6 % faster k_update)
 
 // S_c = sum of the face spectral terms in CSR order, loads issued a chunk at a time
-template <class T>
-__device__ __forceinline__ T spectral_sum(const int* __restrict__ inc, const T* __restrict__ sface, int b, int e) {
-    T s = T(0);
-    constexpr int U = kUpdChunk<T>;
+__device__ __forceinline__ double spectral_sum(const int* __restrict__ inc, const double* __restrict__ sface, int b, int e,
+                                               const Fp& fp) {
+    double s = 0.0;
+    constexpr int U = kUpdChunk;
     for (int i0 = b; i0 < e; i0 += U) {
-        T v[U];
+        double v[U];
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (i0 + u < e) v[u] = sface[inc[i0 + u] >> 1];
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (i0 + u < e) s += v[u];
+            if (i0 + u < e) s = fp.add(s, v[u]);
     }
     return s;
 }
@@ -724,23 +767,23 @@ __device__ __forceinline__ bool positive<double>(double x) {
     return (unsigned long long)__double_as_longlong(x) - 1ull < 0x7ff0000000000000ull;
 }
 
-template <class T, int STAGE>
-__device__ __forceinline__ T update_cell(int c, const DevMesh<T>& m, const Q4<T>* __restrict__ tface,
-                                         const T* __restrict__ sface, Q4<T>* __restrict__ Qn, Q4<T>* __restrict__ Q1,
-                                         Q4<T>* __restrict__ Q2, T* __restrict__ dt, T* __restrict__ S, T smax,
-                                         Q4<T>* __restrict__ Rout, int* __restrict__ flag, const Consts<T>& k,
-                                         int global_dt, T r[4], Q4<T>* __restrict__ D, Q4<T>* __restrict__ Qlo) {
+template <int STAGE>
+__device__ __forceinline__ double update_cell(int c, const Fp& fp, const DevMesh<double>& m, const Q4<double>* __restrict__ tface,
+                                              const double* __restrict__ sface, Q4<double>* __restrict__ Qn,
+                                              Q4<double>* __restrict__ Q1, Q4<double>* __restrict__ Q2, double* __restrict__ dt,
+                                              double* __restrict__ S, double smax, Q4<double>* __restrict__ Rout,
+                                              int* __restrict__ flag, const Consts<double>& k, int global_dt, double r[4]) {
     const int* __restrict__ inc = m.inc;
-    T snext = T(0);
+    double snext = 0.0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) r[j] = T(0);
+    for (int j = 0; j < 4; j++) r[j] = 0.0;
     const int b = m.inc_off[c], e = m.inc_off[c + 1];
     // chunks of kUpdChunk incidences: every record and face contribution of a chunk is requested
     // before the first is summed (more loads in flight per thread); the sums keep CSR order
-    constexpr int U = kUpdChunk<T>;
+    constexpr int U = kUpdChunk;
     for (int i0 = b; i0 < e; i0 += U) {
         int iv[U];
-        Q4<T> tv[U];
+        Q4<double> tv[U];
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (i0 + u < e) iv[u] = inc[i0 + u];
@@ -751,74 +794,42 @@ __device__ __forceinline__ T update_cell(int c, const DevMesh<T>& m, const Q4<T>
         for (int u = 0; u < U; u++) {
             if (i0 + u < e) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) r[j] += neg_if(tv[u].p[j], iv[u] & 1);   // side 1: r -= t
+                for (int j = 0; j < 4; j++) r[j] = fp.add(r[j], neg_if(tv[u].p[j], iv[u] & 1));   // side 1: r -= t
             }
         }
     }
-    const T vc = m.vol[c];
-    const T yv = m.rvol[c];   // Recip<T>::of(vc), precomputed
+    const double vc = m.vol[c];
+    const Divisor vd(vc, m.rvol[c], fp);   // 1/vol precomputed
 #pragma unroll
-    for (int j = 0; j < 4; j++) r[j] = Recip<T>::div(r[j], vc, yv);
-    if (Rout) { Q4<T> rr; for (int j = 0; j < 4; j++) rr.p[j] = r[j]; Rout[c] = rr; }
-    const Q4<T> qn = ldq(Qn, c);
-    Q4<T> out;
-    T dtc;
+    for (int j = 0; j < 4; j++) r[j] = vd.div(r[j], fp);
+    if (Rout) { Q4<double> rr; for (int j = 0; j < 4; j++) rr.p[j] = r[j]; Rout[c] = rr; }
+    const Q4<double> qn = ldq(Qn, c);
+    Q4<double> out;
+    double dtc;
     if (STAGE == 0) {
         dtc = (k.two_cfl * vc) / (global_dt ? smax : S[c]);
         dt[c] = dtc;
     } else {
         dtc = dt[c];
     }
-    if constexpr (sizeof(T) == 4) {
-        if (D) {
-            Q4<T> d;
-            if (STAGE == 0) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) { d.p[j] = dtc * r[j]; out.p[j] = qn.p[j] + d.p[j]; }
-                D[c] = d;
-                Q1[c] = out;
-            } else if (STAGE == 1) {
-                const Q4<T> d1 = ldq((const Q4<T>*)D, c);
-#pragma unroll
-                for (int j = 0; j < 4; j++) { d.p[j] = T(0.25) * d1.p[j] + T(0.25) * dtc * r[j]; out.p[j] = qn.p[j] + d.p[j]; }
-                D[c] = d;
-                Q2[c] = out;
-            } else {
-                const Q4<T> d2 = ldq((const Q4<T>*)D, c);
-                Q4<T> lo = ldq((const Q4<T>*)Qlo, c);
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const T inc_j = T(2.0 / 3.0) * d2.p[j] + T(2.0 / 3.0) * dtc * r[j];
-                    T s, err;
-                    two_sum(qn.p[j], lo.p[j] + inc_j, s, err);
-                    out.p[j] = s;
-                    lo.p[j] = err;
-                }
-                Qn[c] = out;
-                Qlo[c] = lo;
-                snext = spectral_sum(inc, sface, b, e);
-                S[c] = snext;
-            }
-            if (!positive(out.p[0]) || !positive(out.p[3])) atomicOr(flag, 1);
-            return snext;
-        }
-    }
     if (STAGE == 0) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) out.p[j] = qn.p[j] + dtc * r[j];
+        for (int j = 0; j < 4; j++) out.p[j] = fp.add(qn.p[j], fp.mul(dtc, r[j]));
         Q1[c] = out;
-    } else if (STAGE == 1) {
-        const Q4<T> q1 = ldq(Q1, c);
-#pragma unroll
-        for (int j = 0; j < 4; j++) out.p[j] = T(0.75) * qn.p[j] + T(0.25) * q1.p[j] + T(0.25) * dtc * r[j];
-        Q2[c] = out;
-    } else {
-        const Q4<T> q2 = ldq(Q2, c);
+    } else if (STAGE == 1) {   // 3/4 Qn + 1/4 Q1 + 1/4 dt R, the exact quarters on the multiply-adds
+        const Q4<double> q1 = ldq(Q1, c);
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            out.p[j] = T(1.0 / 3.0) * qn.p[j] + T(2.0 / 3.0) * q2.p[j] + T(2.0 / 3.0) * dtc * r[j];
+            out.p[j] = __fma_rn(fp.mul(dtc, r[j]), 0.25, __fma_rn(q1.p[j], 0.25, fp.mul(0.75, qn.p[j])));
+        Q2[c] = out;
+    } else {
+        const Q4<double> q2 = ldq(Q2, c);
+        const double dt23 = fp.mul(2.0 / 3.0, dtc);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            out.p[j] = fp.add(fp.add(fp.mul(1.0 / 3.0, qn.p[j]), fp.mul(2.0 / 3.0, q2.p[j])), fp.mul(dt23, r[j]));
         Qn[c] = out;
-        snext = spectral_sum(inc, sface, b, e);
+        snext = spectral_sum(inc, sface, b, e, fp);
         S[c] = snext;
     }
     if (!positive(out.p[0]) || !positive(out.p[3])) atomicOr(flag, 1);
@@ -828,21 +839,22 @@ __device__ __forceinline__ T update_cell(int c, const DevMesh<T>& m, const Q4<T>
 #ifndef FV2D_UPD_BLOCK
 #define FV2D_UPD_BLOCK 256   // threads per block of the single-solve update kernel
 #endif
-template <class T, int STAGE>
+template <int STAGE>
 __global__ void __launch_bounds__(FV2D_UPD_BLOCK)
-k_update(int nc, DevMesh<T> m, const Q4<T>* __restrict__ tface, const T* __restrict__ sface, Q4<T>* __restrict__ Qn,
-         Q4<T>* __restrict__ Q1, Q4<T>* __restrict__ Q2, T* __restrict__ dt, T* __restrict__ S, T* __restrict__ smax,
-         Q4<T>* __restrict__ Rout, int* __restrict__ flag, Consts<T> k, int global_dt, Q4<T>* __restrict__ D,
-         Q4<T>* __restrict__ Qlo) {
+k_update(int nc, DevMesh<double> m, const Q4<double>* __restrict__ tface, const double* __restrict__ sface,
+         Q4<double>* __restrict__ Qn, Q4<double>* __restrict__ Q1, Q4<double>* __restrict__ Q2, double* __restrict__ dt,
+         double* __restrict__ S, double* __restrict__ smax, Q4<double>* __restrict__ Rout, int* __restrict__ flag,
+         Consts<double> k, int global_dt) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    T snext = T(0);
+    double snext = 0.0;
     if (c < nc) {
-        T r[4];
-        snext = update_cell<T, STAGE>(c, m, tface, sface, Qn, Q1, Q2, dt, S, (STAGE == 0 && global_dt) ? *smax : T(0),
-                                      Rout, flag, k, global_dt, r, D, Qlo);
+        const Fp fp;
+        double r[4];
+        snext = update_cell<STAGE>(c, fp, m, tface, sface, Qn, Q1, Q2, dt, S, (STAGE == 0 && global_dt) ? *smax : 0.0, Rout, flag,
+                                   k, global_dt, r);
     }
     if (STAGE == 2) {
-        const T mx = block_max(c < nc ? snext : T(0));
+        const double mx = block_max(c < nc ? snext : 0.0);
         if (threadIdx.x == 0) atomic_max_pos(smax, mx);
     }
 }

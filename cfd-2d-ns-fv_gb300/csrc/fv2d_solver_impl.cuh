@@ -201,26 +201,26 @@ public:
         Q4<T>* qin = Q_[s];
         const int p = (s + 2) % 3;
         if (order2_) {
-            constexpr int B = kStageBlock<T>;
+            constexpr int B = FV2D_FP64_BLOCK;
             launch(K_GRADIENT, nc_, [&](int gr) {
                 if (squeeze_)
-                    k_gradient<T, true><<<gr, B, 0, stream_>>>(nc_, dm_, qin, Q_[p], G_[p], G_[s], k_, fresh_ ? 1 : 0,
+                    k_gradient<true><<<gr, B, 0, stream_>>>(nc_, dm_, qin, Q_[p], G_[p], G_[s], k_, fresh_ ? 1 : 0,
                                                               init_prims_ ? 1 : 0);
                 else
-                    k_gradient<T, false><<<gr, B, 0, stream_>>>(nc_, dm_, qin, Q_[p], G_[p], G_[s], k_, fresh_ ? 1 : 0,
+                    k_gradient<false><<<gr, B, 0, stream_>>>(nc_, dm_, qin, Q_[p], G_[p], G_[s], k_, fresh_ ? 1 : 0,
                                                                init_prims_ ? 1 : 0);
             }, B);
         }
-        launch(K_FACE, nf_, [&](int gr) { launch_face(gr, qin, G_[s], s == 2); }, kStageBlock<T>);
+        launch(K_FACE, nf_, [&](int gr) { launch_face(gr, qin, G_[s], s == 2); }, FV2D_FP64_BLOCK);
         if (s == 2) FV2D_CUDA(cudaMemsetAsync(smax_, 0, sizeof(T), stream_));
         Q4<T>* rout = (store_every_ || s == 2) ? R_ : nullptr;
         launch(K_UPDATE, nc_, [&](int gr) {
             if (s == 0)
-                k_update<T, 0><<<gr, FV2D_UPD_BLOCK, 0, stream_>>>(nc_, dm_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout, flag_, k_, global_dt_, D_, Qlo_);
+                k_update<0><<<gr, FV2D_UPD_BLOCK, 0, stream_>>>(nc_, dm_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout, flag_, k_, global_dt_);
             else if (s == 1)
-                k_update<T, 1><<<gr, FV2D_UPD_BLOCK, 0, stream_>>>(nc_, dm_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout, flag_, k_, global_dt_, D_, Qlo_);
+                k_update<1><<<gr, FV2D_UPD_BLOCK, 0, stream_>>>(nc_, dm_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout, flag_, k_, global_dt_);
             else
-                k_update<T, 2><<<gr, FV2D_UPD_BLOCK, 0, stream_>>>(nc_, dm_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout, flag_, k_, global_dt_, D_, Qlo_);
+                k_update<2><<<gr, FV2D_UPD_BLOCK, 0, stream_>>>(nc_, dm_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout, flag_, k_, global_dt_);
         }, FV2D_UPD_BLOCK);
         FV2D_CUDA(cudaGetLastError());
         if (s == 0) { fresh_ = false; init_prims_ = false; }
@@ -352,7 +352,7 @@ public:
 private:
     void launch_face(int gr, const Q4<T>* qin, const Q4<T>* G, bool last) {
 #define FV2D_FACE(O2, NS, LAST) \
-    k_face<T, O2, NS, LAST><<<gr, kStageBlock<T>, 0, stream_>>>(nf_, dm_, qin, G, t_, s_, k_, init_prims_ ? 1 : 0)
+    k_face<O2, NS, LAST><<<gr, FV2D_FP64_BLOCK, 0, stream_>>>(nf_, dm_, qin, G, t_, s_, k_, init_prims_ ? 1 : 0)
         if (order2_) {
             if (ns_) { if (last) FV2D_FACE(true, true, true); else FV2D_FACE(true, true, false); }
             else { if (last) FV2D_FACE(true, false, true); else FV2D_FACE(true, false, false); }
