@@ -39,20 +39,6 @@ struct Tile {
 };
 
 template <class T>
-__device__ __forceinline__ T block_sum(T v, T* red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) red[w] = v;
-    __syncthreads();
-    T s = T(0);
-    if (threadIdx.x == 0)
-        for (int i = 0; i < (int)(blockDim.x >> 5); i++) s += red[i];
-    return s;   // valid in thread 0
-}
-
-template <class T>
 __device__ __forceinline__ T block_max_t(T v, T* red) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = max2(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -65,10 +51,6 @@ __device__ __forceinline__ T block_max_t(T v, T* red) {
         for (int i = 0; i < (int)(blockDim.x >> 5); i++) s = max2(s, red[i]);
     return s;   // valid in thread 0
 }
-
-#ifndef FV2D_BATCH_FVAL
-#define FV2D_BATCH_FVAL 1   // FP64 batches store the face states for the limiter (0: recompute them)
-#endif
 
 // Largest block the batch kernels accept (the autotuner's largest) and the FP32 kernels' minimum
 // resident blocks at that size (their register caps: gradient 64, face 48 - measured fastest);
@@ -87,8 +69,7 @@ constexpr int kBatchMinB64 = 512 / FV2D_KB_MAXT;
 template <class T>
 __global__ void __launch_bounds__(FV2D_KB_MAXT, sizeof(T) == 4 ? FV2D_KBG_MINB32 : FV2D_KBG_MINB64)
 kb_gradient(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevMesh<T> m,
-            const SolveParams<T>* __restrict__ P, const Q4<T>* __restrict__ Qin, const Q4<T>* __restrict__ Qprev,
-            const Q4<T>* __restrict__ Gprev, Q4<T>* __restrict__ Gout) {
+            const SolveParams<T>* __restrict__ P, const Q4<T>* __restrict__ Qin, Q4<T>* __restrict__ Gout) {
     __shared__ SolveParams<T> sp;
     __shared__ Tile st;
     const Fp fp;
@@ -96,14 +77,11 @@ kb_gradient(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevM
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         if (threadIdx.x == 0) { st = tiles[t]; sp = P[st.sid]; }
         __syncthreads();
-        if (sp.order2) {
-            if (sp.squeeze) {
-                for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                    gradient_cell<true, true, FV2D_KB_MAXT / 32>(st.start + e, fp, m, Qin, Qprev, Gprev, Gout, sp.k,
-                                                                             sp.fresh, sp.init_prims);
-            } else {
-                for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                    gradient_cell<false>(st.start + e, fp, m, Qin, Qprev, Gprev, Gout, sp.k, sp.fresh, sp.init_prims);
+        if (sp.order2) {   // four lanes (one component each) per cell
+            const int j = threadIdx.x & 3;
+            for (int e = threadIdx.x >> 2; e < st.count; e += blockDim.x >> 2) {
+                if (sp.squeeze) gradient_lane<true>(st.start + e, j, fp, m, Qin, Gout, sp.k, sp.fresh, sp.init_prims, NoWait());
+                else gradient_lane<false>(st.start + e, j, fp, m, Qin, Gout, sp.k, sp.fresh, sp.init_prims, NoWait());
             }
         }
         __syncthreads();
@@ -127,13 +105,13 @@ kb_face(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevMesh<
         __syncthreads();
         if (!sp.order2) {
             for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                face_flux<false, false, LAST>(st.start + e, fp, m, Qin, G, tout, sout, sp.k, sp.init_prims);
+                face_flux<false, false, LAST>(st.start + e, fp, m, Qin, G, tout, sout, sp.k, sp.init_prims, NoWait());
         } else if (sp.ns) {
             for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                face_flux<true, true, LAST>(st.start + e, fp, m, Qin, G, tout, sout, sp.k, sp.init_prims);
+                face_flux<true, true, LAST>(st.start + e, fp, m, Qin, G, tout, sout, sp.k, sp.init_prims, NoWait());
         } else {
             for (int e = threadIdx.x; e < st.count; e += blockDim.x)
-                face_flux<true, false, LAST>(st.start + e, fp, m, Qin, G, tout, sout, sp.k, sp.init_prims);
+                face_flux<true, false, LAST>(st.start + e, fp, m, Qin, G, tout, sout, sp.k, sp.init_prims, NoWait());
         }
         __syncthreads();
     }
@@ -144,36 +122,53 @@ __global__ void __launch_bounds__(FV2D_KB_MAXT)
 kb_update(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevMesh<T> m, SolveParams<T>* P,
           const Q4<T>* __restrict__ tface, const T* __restrict__ sface, Q4<T>* __restrict__ Qn, Q4<T>* __restrict__ Q1,
           Q4<T>* __restrict__ Q2, T* __restrict__ dt, T* __restrict__ S, T* __restrict__ smax, double* __restrict__ tpart,
-          int* __restrict__ flags, Q4<T>* __restrict__ D, Q4<T>* __restrict__ Qlo) {
+          int* __restrict__ flags) {
     __shared__ SolveParams<T> sp;
     __shared__ Tile st;
-    __shared__ double redd[32];
+    __shared__ double redd[32][4];
     __shared__ T redt[32];
     const Fp fp;
     const int nt = *ntiles;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         if (threadIdx.x == 0) { st = tiles[t]; sp = P[st.sid]; }
         __syncthreads();
-        const T sm = (STAGE == 0 && sp.global_dt) ? smax[st.sid] : T(0);
-        T mx = T(0);
-        double acc[4] = {0, 0, 0, 0};
-        for (int e = threadIdx.x; e < st.count; e += blockDim.x) {
-            T r[4];
-            const T sn = update_cell<STAGE>(st.start + e, fp, m, tface, sface, Qn, Q1, Q2, dt, S, sm, nullptr,
-                                               flags + st.sid, sp.k, sp.global_dt, r);
-            if (STAGE == 2) {
-                mx = max2(mx, sn);
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[j] += (double)r[j] * (double)r[j];
+        // four lanes (one component each) per cell; what a cell needs once (its time step in the first
+        // stage, its spectral sum in the last) takes one lane per cell
+        if (STAGE == 0) {
+            const T sm = sp.global_dt ? smax[st.sid] : T(0);
+            for (int e = threadIdx.x; e < st.count; e += blockDim.x) {
+                const int c = st.start + e;
+                dt[c] = (sp.k.two_cfl * m.vol[c]) / (sp.global_dt ? sm : S[c]);
             }
+            __syncthreads();
+        }
+        double acc = 0.0;
+        const int j = threadIdx.x & 3;
+        for (int e = threadIdx.x >> 2; e < st.count; e += blockDim.x >> 2) {
+            const double r = update_lane<STAGE>(st.start + e, j, fp, m, UpdateMesh(st.start + e, m), tface, Qn, Q1, Q2,
+                                                dt[st.start + e], nullptr, flags + st.sid);
+            if (STAGE == 2) acc = fp.add(acc, fp.mul(r, r));
         }
         if (STAGE == 2) {
+            T mx = T(0);
+            for (int e = threadIdx.x; e < st.count; e += blockDim.x) {
+                const int c = st.start + e;
+                const T sn = spectral_sum(m.inc, sface, m.inc_off[c], m.inc_off[c + 1], fp);
+                S[c] = sn;
+                mx = max2(mx, sn);
+            }
             const T bm = block_max_t(mx, redt);
             if (threadIdx.x == 0) atomic_max_pos(smax + st.sid, bm);
+            // the tile's sum of squares per component: over the lanes of a component in each warp, then over
+            // the warps in order
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const double bs = block_sum(acc[j], redd);
-                if (threadIdx.x == 0) tpart[4 * (size_t)t + j] = bs;   // this tile's sum of squares
+            for (int o = 16; o >= 4; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if ((threadIdx.x & 31) < 4) redd[threadIdx.x >> 5][j] = acc;
+            __syncthreads();
+            if (threadIdx.x < 4) {
+                double s = 0.0;
+                for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += redd[w][threadIdx.x];
+                tpart[4 * (size_t)t + threadIdx.x] = s;
             }
         }
         if (STAGE == 0 && threadIdx.x == 0) { P[st.sid].fresh = 0; P[st.sid].init_prims = 0; }
@@ -302,7 +297,7 @@ public:
         size_t oD = comp ? take(q4 * Nc_) : 0, olo = comp ? take(q4 * Nc_) : 0;
         // FP64: the face pass stores its reconstructed face states for the next squeeze (as the
         // single-solve FP64 engine does); a solve's first stage after admission uses the sentinel
-        const bool fv = !comp && FV2D_BATCH_FVAL;
+        const bool fv = !comp;
         size_t ofval = fv ? take(2 * q4 * Fc_) : 0;
         tile_cap_ = (int)std::min<long long>((Nc_ + Fc_) / 64 + 4 * (long long)S_ + 16, 1LL << 28);
         size_t otc = take(sizeof(Tile) * tile_cap_), otf = take(sizeof(Tile) * tile_cap_), ocnt = take(64);
@@ -702,9 +697,8 @@ private:
         const int* nct = cnt_;
         const int* nft = cnt_ + 1;
         for (int s = 0; s < 3; s++) {
-            const int p = (s + 2) % 3;
             timed(0, [&] {
-                kb_gradient<T><<<gg_, B, 0, stream_>>>(tc_, nct, m_, P_, Q_[s], Q_[p], G_[p], G_[s]);
+                kb_gradient<T><<<gg_, B, 0, stream_>>>(tc_, nct, m_, P_, Q_[s], G_[s]);
             });
             timed(1, [&] {
                 if (s == 2)
@@ -715,11 +709,11 @@ private:
             if (s == 2) FV2D_B(cudaMemsetAsync(smax_, 0, sizeof(T) * S_, stream_));
             timed(2, [&] {
                 if (s == 0)
-                    kb_update<T, 0><<<gu_[0], B, 0, stream_>>>(tc_, nct, m_, P_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_arr_, smax_, tpart_, flags_, D_, Qlo_);
+                    kb_update<T, 0><<<gu_[0], B, 0, stream_>>>(tc_, nct, m_, P_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_arr_, smax_, tpart_, flags_);
                 else if (s == 1)
-                    kb_update<T, 1><<<gu_[1], B, 0, stream_>>>(tc_, nct, m_, P_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_arr_, smax_, tpart_, flags_, D_, Qlo_);
+                    kb_update<T, 1><<<gu_[1], B, 0, stream_>>>(tc_, nct, m_, P_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_arr_, smax_, tpart_, flags_);
                 else
-                    kb_update<T, 2><<<gu_[2], B, 0, stream_>>>(tc_, nct, m_, P_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_arr_, smax_, tpart_, flags_, D_, Qlo_);
+                    kb_update<T, 2><<<gu_[2], B, 0, stream_>>>(tc_, nct, m_, P_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_arr_, smax_, tpart_, flags_);
             });
             if (s == 2) kb_res_norm<T><<<S_, 256, 0, stream_>>>(srange_, tpart_, res2_);
             FV2D_B(cudaGetLastError());

@@ -61,9 +61,24 @@ struct DevMesh {
 };
 
 template <class T>
-__device__ __forceinline__ Q4<T> ldq(const Q4<T>* __restrict__ a, int i) {
+__device__ __forceinline__ Q4<T> ldq(const Q4<T>* a, int i) {
     return a[i];
 }
+
+// Programmatic dependent launch: a stage kernel loads what no kernel writes (the mesh), waits for the
+// kernel before it and then lets the next one's CTAs start.  So at most two kernels are in flight, and
+// a waiting kernel's SM reads nothing that the running one writes.  (The arrays that kernels write are
+// not __restrict__ const: they change while a waiting kernel is resident, so its loads of them must not
+// go by the read-only path.)
+struct Prior {
+    __device__ __forceinline__ void operator()() const {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+};
+struct NoWait {
+    __device__ __forceinline__ void operator()() const {}
+};
 
 // Ordered comparison a < b.  For doubles it runs on the integer pipe: a non-NaN double's bit
 // pattern, with -0 folded onto +0 and the magnitude bits of negatives inverted, orders exactly as
@@ -235,257 +250,147 @@ __device__ __forceinline__ T pick4(const T a[4], int j) {
 }
 
 #ifndef FV2D_FP64_BLOCK
-#define FV2D_FP64_BLOCK 128   // threads per block of the FP64 gradient and face kernels
+#define FV2D_FP64_BLOCK 128   // threads per block of the gradient and face kernels
 #endif
 
-// Shared-memory staging of the warp-shared limiter quotients (FP64 single solve, see gradient_cell)
-#ifndef FV2D_WARPQ_CAP
-#define FV2D_WARPQ_CAP 256   // flagged checks per warp held at once; warps with more use the per-cell loop
-#endif
-template <int WARPS>
-struct WarpQ {
-    double qc[WARPS][4][32], mn[WARPS][4][32], mx[WARPS][4][32];   // each cell's state and bounds
-    int b[WARPS][32];                                               // each cell's first incidence
-    unsigned short list[WARPS][FV2D_WARPQ_CAP];                     // (lane << 6) | check bit
-    double quo[WARPS][FV2D_WARPQ_CAP];                              // the checks' quotients
-};
-
-template <bool SQUEEZE, bool WARPQ = false, int QWARPS = FV2D_FP64_BLOCK / 32>
-__device__ __forceinline__ void gradient_cell(int c, const Fp& fp, const DevMesh<double>& m, const Q4<double>* __restrict__ Q,
-                                              const Q4<double>* __restrict__ Qprev, const Q4<double>* __restrict__ Gprev,
-                                              Q4<double>* __restrict__ Gout, const Consts<double>& k, int first_stage,
-                                              int init_prims) {
-    using T = double;
-    const int* __restrict__ inc_off = m.inc_off;
+// One component j of cell c's limited gradient: a thread per cell and component.  The components share
+// only the mesh and, at walls, the ghost's primitives, so four lanes per cell do the same FP64 work
+// as one, in a quarter of the chain (64 cycles an operation for a lone warp, whatever its active
+// lanes) and with fewer registers.  With the limiter below: 8,192 quads 107 -> 67 us per iteration, 50k NS
+// polygons 446 -> 395, 400k 2,854 -> 2,752 (update_lane's share included).
+// The limiter takes the smallest of 1 and the factors (bound - Q) / (face value - Q) of the previous face
+// values that leave the bounds (squeeze.cpp:68-141).  Rounded subtraction and division are monotone, so
+// on either side the smallest factor is the one at the extreme face value: one division per
+// violated side instead of one per violating face.  Where the bounds meet (the neighbourhood is uniform)
+// every factor is a zero, -0 below and +0 above, and the reference keeps the last face's.
+template <bool SQUEEZE, class Wait>
+__device__ __forceinline__ void gradient_lane(int c, int j, const Fp& fp, const DevMesh<double>& m, const Q4<double>* Q,
+                                              Q4<double>* Gout, const Consts<double>& k, int first_stage, int init_prims, Wait wait) {
     const int* __restrict__ inc = m.inc;
     const int* __restrict__ nbr = m.nbr;
-    const int* __restrict__ qcell = m.qcell;
-    const FaceGeo<T>& g = m.g;
-    const Q4<T> qc = ldq(Q, c);
-    T sx[4] = {T(0), T(0), T(0), T(0)}, sy[4] = {T(0), T(0), T(0), T(0)};
-    T qmin[4], qmax[4];
-    if (SQUEEZE)
-        for (int j = 0; j < 4; j++) { qmin[j] = T(100000000000.0); qmax[j] = T(-100000000000.0); }
-    const int b = inc_off[c], e = inc_off[c + 1];
-    // software-pipelined: the next incidence's record and neighbour state are requested before
-    // the current one is processed (every cell has at least 3 faces, so entry b exists)
-    int inc_n = inc[b], nb_n = nbr[b];
-    Q4<T> ig_n = ldq(m.igeo, b), qn_n;
-    if (nb_n >= 0) qn_n = ldq(Q, nb_n);
+    const double* Qd = reinterpret_cast<const double*>(Q);
+    const double* fv = reinterpret_cast<const double*>(m.fval);
+    const FaceGeo<double>& g = m.g;
+    const int b = m.inc_off[c], e = m.inc_off[c + 1];
+    double sx = 0.0, sy = 0.0;
+    // software-pipelined: the ids of the incidence after next and the states of the next one are
+    // requested before the current one is processed (every cell has at least 3 faces)
+    int inc_n = inc[b], nb_n = nbr[b], inc_2 = inc[b + 1], nb_2 = nbr[b + 1];
+    double2 ig_n = *reinterpret_cast<const double2*>(m.igeo + b);
+    wait();
+    const double qc = Qd[4 * (size_t)c + j];
+    double qn_n = 0.0, qf_n = -101.0;   // -101: the face states before the first stage (class_q.hpp:73-76)
+    auto states = [&] {
+        if (nb_n >= 0) qn_n = Qd[4 * (size_t)nb_n + j];
+        if (SQUEEZE && !first_stage) qf_n = fv[4 * (size_t)inc_n + j];
+    };
+    states();
+    // the bounds start with the first face's states in the reference's order (squeeze.cpp: the c1
+    // side's, then the c2 side's), which decides between +0 and -0
+    double mn = qc, mx = qc, fmn = 0.0, fmx = 0.0;
+    long long kc = 0, kmn = 0, kmx = 0, kfmn = 0, kfmx = 0;
+    int last = 0;   // the last face value that differs from Q: below (-1) or above (1)
+    if (SQUEEZE) {
+        kc = order_key(qc);
+        if (nb_n >= 0 && (inc_n & 1)) mn = mx = qn_n;
+        kmn = kmx = order_key(mn);
+        if (kc < kmn) { kmn = kc; mn = qc; }
+        if (kmx < kc) { kmx = kc; mx = qc; }
+        fmn = fmx = qf_n;
+        kfmn = kfmx = order_key(qf_n);
+    }
     for (int i = b; i < e; i++) {
         const int f = inc_n >> 1, side = inc_n & 1, nb = nb_n;
-        const Q4<T> ig = ig_n, qn = qn_n;
+        const double2 ig = ig_n;
+        const double qn = qn_n, qf = qf_n;
         if (i + 1 < e) {
-            inc_n = inc[i + 1];
-            nb_n = nbr[i + 1];
-            ig_n = ldq(m.igeo, i + 1);
-            if (nb_n >= 0) qn_n = ldq(Q, nb_n);
+            inc_n = inc_2;
+            nb_n = nb_2;
+            ig_n = *reinterpret_cast<const double2*>(m.igeo + i + 1);
+            states();
+            if (i + 2 < e) { inc_2 = inc[i + 2]; nb_2 = nbr[i + 2]; }
         }
-        T d[4];
+        double d;
         if (nb >= 0) {
-            const T* q1 = side == 0 ? qc.p : qn.p;   // reference orientation: c2 - c1
-            const T* q2 = side == 0 ? qn.p : qc.p;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                d[j] = fp.sub(q2[j], q1[j]);
-                if (SQUEEZE) {
-                    qmin[j] = min2(qmin[j], min2(q1[j], q2[j]));
-                    qmax[j] = max2(qmax[j], max2(q1[j], q2[j]));
-                }
+            d = side == 0 ? fp.sub(qn, qc) : fp.sub(qc, qn);   // reference orientation: c2 - c1
+            if (SQUEEZE) {
+                const long long kn = order_key(qn);
+                if (kn < kmn) { kmn = kn; mn = qn; }
+                if (kmx < kn) { kmx = kn; mx = qn; }
             }
+        } else if (nb == -1) {
+            d = fp.sub(pick4(k.q_inf, j), qc);
+        } else if (nb == -2 || nb == -4) {
+            double rho, u, v, P, gq[4];
+            if (init_prims) { rho = k.rho_inf; u = k.u_inf; v = k.v_inf; P = k.P_inf; }
+            else {
+                const Q4<double> qq = Q[nb == -2 ? c : m.qcell[f]];
+                rho = qq.p[0];
+                prims_r(qq.p, k, fp, u, v, P);
+            }
+            if (nb == -2) {        // slip wall: reflect the cell velocity (cell_gradient.cpp:43-55)
+                const double fnx = g.nx[f], fny = g.ny[f];
+                const double vn = u * fnx + v * fny;
+                cons(rho, u - 2.0 * vn * fnx, v - 2.0 * vn * fny, P, k, gq);
+            } else {               // no-slip: state of cell `face id`, velocity negated (:62-73)
+                cons(rho, -u, -v, P, k, gq);
+            }
+            d = fp.sub(pick4(gq, j), qc);
         } else {
-            if (nb == -1) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) d[j] = fp.sub(k.q_inf[j], qc.p[j]);
-            } else if (nb == -2 || nb == -4) {
-                T rho, u, v, P;
-                if (init_prims) { rho = k.rho_inf; u = k.u_inf; v = k.v_inf; P = k.P_inf; }
-                else if (nb == -2) { rho = qc.p[0]; prims_r(qc.p, k, fp, u, v, P); }
-                else { const Q4<T> qq = ldq(Q, qcell[f]); rho = qq.p[0]; prims_r(qq.p, k, fp, u, v, P); }
-                T gq[4];
-                if (nb == -2) {        // slip wall: reflect the cell velocity (cell_gradient.cpp:43-55)
-                    const T fnx = g.nx[f], fny = g.ny[f];
-                    const T vn = u * fnx + v * fny;
-                    cons(rho, u - T(2.0) * vn * fnx, v - T(2.0) * vn * fny, P, k, gq);
-                } else {               // no-slip: state of cell `face id`, velocity negated (:62-73)
-                    cons(rho, -u, -v, P, k, gq);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) d[j] = fp.sub(gq[j], qc.p[j]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) d[j] = T(0);
-            }
-            if (SQUEEZE)
-#pragma unroll
-                for (int j = 0; j < 4; j++) { qmin[j] = min2(qmin[j], qc.p[j]); qmax[j] = max2(qmax[j], qc.p[j]); }
+            d = 0.0;
         }
-        const T fx = ig.p[0], fy = ig.p[1];
-#pragma unroll
-        for (int j = 0; j < 4; j++) { sx[j] = fp.add(sx[j], fp.mul(d[j], fx)); sy[j] = fp.add(sy[j], fp.mul(d[j], fy)); }
+        if (SQUEEZE) {
+            const long long kf = order_key(qf);
+            if (kf < kfmn) { kfmn = kf; fmn = qf; }
+            if (kfmx < kf) { kfmx = kf; fmx = qf; }
+            last = kf < kc ? -1 : kc < kf ? 1 : last;
+        }
+        sx = fp.add(sx, fp.mul(d, ig.x));
+        sy = fp.add(sy, fp.mul(d, ig.y));
     }
-    const T ixx = (T)m.Ixx[c], iyy = (T)m.Iyy[c], ixy = (T)m.Ixy[c];
-    Q4<T> gx, gy;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        gx.p[j] = fp.sub(fp.mul(sx[j], iyy), fp.mul(sy[j], ixy));
-        gy.p[j] = fp.sub(fp.mul(sy[j], ixx), fp.mul(sx[j], ixy));
-    }
+    const double ixx = m.Ixx[c], iyy = m.Iyy[c], ixy = m.Ixy[c];
+    double gx = fp.sub(fp.mul(sx, iyy), fp.mul(sy, ixy));
+    double gy = fp.sub(fp.mul(sy, ixx), fp.mul(sx, ixy));
     if (SQUEEZE) {
-        T phi[4] = {T(1), T(1), T(1), T(1)};
-        Q4<T> qp, gpx, gpy;
-        const Q4<T>* __restrict__ fval = m.fval;
-        if (!first_stage && !fval) { qp = ldq(Qprev, c); gpx = ldq(Gprev, 2 * c); gpy = ldq(Gprev, 2 * c + 1); }
-        {
-            // Only a minority of the (incidence, component) checks bound the face value and
-            // need a quotient, but a conditional IEEE division is if-converted (computed for every
-            // check).  So one pass flags the checks that need one (bit 4*(incidence - i0) + component,
-            // 16 incidences per word) and a second loop takes one flagged check per trip - one
-            // division per trip, so a warp runs as many divisions as its busiest cell has flags -
-            // in ascending bit order, so every min2 applies in the original sequence per component.
-            // An unflagged check's factor 1 leaves phi unchanged bit for bit (phi <= 1).
-            // WARPQ (FP64 single solve, stored face states): a warp's flagged checks are listed in
-            // shared memory and spread over its 32 lanes, one quotient per lane per round, so the
-            // warp runs ceil(flagged / 32) divisions instead of its busiest cell's count; each cell
-            // then applies its own quotients in ascending bit order, as the loop below does.
-            bool shared_done = false;
-            if constexpr (WARPQ) {
-                constexpr unsigned FULL = 0xffffffffu;
-                // taken by the whole warp or by none of it (the shuffles below need all 32 lanes):
-                // a converged full warp whose cells all have at most 16 faces, in a block no larger
-                // than the one the shared staging is sized for (QWARPS warps)
-                if (fval != nullptr && blockDim.x <= 32 * QWARPS && __activemask() == FULL &&
-                    __all_sync(FULL, e - b <= 16)) {
-                    unsigned long long mask = 0;
-                    for (int i = b; i < e; i++) {
-                        Q4<T> qf;
-                        if (first_stage) {
-#pragma unroll
-                            for (int j = 0; j < 4; j++) qf.p[j] = T(-101);
-                        } else {
-                            qf = ldq(fval, inc[i]);
-                        }
-#pragma unroll
-                        for (int j = 0; j < 4; j++)
-                            if (less(qf.p[j], qmin[j]) || less(qmax[j], qf.p[j])) mask |= 1ull << (4 * (i - b) + j);
-                    }
-                    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-                    const int cnt = __popcll(mask);
-                    int incl = cnt;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int v = __shfl_up_sync(FULL, incl, o);
-                        if (lane >= o) incl += v;
-                    }
-                    const int total = __shfl_sync(FULL, incl, 31), excl = incl - cnt;
-                    if (total <= FV2D_WARPQ_CAP) {
-                        __shared__ WarpQ<QWARPS> sq;
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            sq.qc[w][j][lane] = qc.p[j];
-                            sq.mn[w][j][lane] = qmin[j];
-                            sq.mx[w][j][lane] = qmax[j];
-                        }
-                        sq.b[w][lane] = b;
-                        {
-                            unsigned long long mm = mask;
-                            int pos = excl;
-                            while (mm) {
-                                const int bit = __ffsll((long long)mm) - 1;
-                                mm &= mm - 1;
-                                sq.list[w][pos++] = (unsigned short)((lane << 6) | bit);
-                            }
-                        }
-                        __syncwarp();
-                        for (int g = lane; g < total; g += 32) {
-                            const int ent = sq.list[w][g], ow = ent >> 6, bit = ent & 63, j = bit & 3;
-                            const T qf = first_stage ? T(-101)
-                                                     : reinterpret_cast<const T*>(fval)[4 * (size_t)inc[sq.b[w][ow] + (bit >> 2)] + j];
-                            const T qcj = sq.qc[w][j][ow], mn = sq.mn[w][j][ow], mx = sq.mx[w][j][ow];
-                            const T num = less(qf, mn) ? mn : mx;
-                            sq.quo[w][g] = (num - qcj) / (qf - qcj);
-                        }
-                        __syncwarp();
-                        {
-                            unsigned long long mm = mask;
-                            int pos = excl;
-                            while (mm) {
-                                const int bit = __ffsll((long long)mm) - 1;
-                                mm &= mm - 1;
-                                const int j = bit & 3;
-                                const T ph = min2((T)sq.quo[w][pos++], pick4(phi, j));
-#pragma unroll
-                                for (int jj = 0; jj < 4; jj++) phi[jj] = jj == j ? ph : phi[jj];
-                            }
-                        }
-                        __syncwarp();
-                        shared_done = true;
-                    }
-                }
+        // the reference's starting values
+        if (!(kmn < order_key(100000000000.0))) { mn = 100000000000.0; kmn = order_key(mn); }
+        if (!(order_key(-100000000000.0) < kmx)) { mx = -100000000000.0; kmx = order_key(mx); }
+        const bool below = kfmn < kmn, above = kmx < kfmx;
+        double phi = 1.0;
+        if (below || above) {   // one division for the violated side, a second where both are
+            phi = fp.sub(below ? mn : mx, qc) / fp.sub(below ? fmn : fmx, qc);
+            if (below && above) {
+                const double up = fp.sub(mx, qc) / fp.sub(fmx, qc);
+                const bool zeros = ((__double_as_longlong(phi) | __double_as_longlong(up)) << 1) == 0;
+                phi = zeros ? (last < 0 ? phi : up) : min2(up, phi);
             }
-            for (int i0 = b; i0 < (shared_done ? b : e); i0 += 16) {
-                const int i1 = min(e, i0 + 16);
-                unsigned long long mask = 0;
-                for (int i = i0; i < i1; i++) {
-                    Q4<T> qf;
-                    if (first_stage) {
-#pragma unroll
-                        for (int j = 0; j < 4; j++) qf.p[j] = T(-101);
-                    } else if (fval) {
-                        qf = ldq(fval, inc[i]);
-                    } else {
-                        const Q4<T> ig = ldq(m.igeo, i);
-#pragma unroll
-                        for (int j = 0; j < 4; j++) qf.p[j] = qp.p[j] + gpx.p[j] * ig.p[2] + gpy.p[j] * ig.p[3];
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        if (less(qf.p[j], qmin[j]) || less(qmax[j], qf.p[j])) mask |= 1ull << (4 * (i - i0) + j);
-                }
-                while (mask) {
-                    const int bit = __ffsll((long long)mask) - 1;
-                    mask &= mask - 1;
-                    const int j = bit & 3, i = i0 + (bit >> 2);
-                    const T qcj = pick4(qc.p, j), mn = pick4(qmin, j), mx = pick4(qmax, j);
-                    T qf;
-                    if (first_stage) qf = T(-101);
-                    else if (fval) qf = reinterpret_cast<const T*>(fval)[4 * (size_t)inc[i] + j];
-                    else {
-                        const Q4<T> ig = ldq(m.igeo, i);
-                        qf = pick4(qp.p, j) + pick4(gpx.p, j) * ig.p[2] + pick4(gpy.p, j) * ig.p[3];
-                    }
-                    const T num = less(qf, mn) ? mn : mx;
-                    const T ph = min2((num - qcj) / (qf - qcj), pick4(phi, j));
-#pragma unroll
-                    for (int jj = 0; jj < 4; jj++) phi[jj] = jj == j ? ph : phi[jj];
-                }
-            }
+            phi = min2(phi, 1.0);
         }
-#pragma unroll
-        for (int j = 0; j < 4; j++) { gx.p[j] = fp.mul(gx.p[j], phi[j]); gy.p[j] = fp.mul(gy.p[j], phi[j]); }
+        gx = fp.mul(gx, phi);
+        gy = fp.mul(gy, phi);
     }
-    Gout[2 * c] = gx;
-    Gout[2 * c + 1] = gy;
+    double* go = reinterpret_cast<double*>(Gout + 2 * (size_t)c);
+    go[j] = gx;
+    go[4 + j] = gy;
 }
 
-// Occupancy: the kernels are FP64-pipe-bound; their block size and minimum resident blocks (register
-// cap) set how many warps cover the pipe's latency.
 #ifndef FV2D_FP64_GMINB
-#define FV2D_FP64_GMINB 8   // 8 x 128 threads at 64 registers (spilling), 8 x 23 KB of shared memory:
-                            // 4 % faster than half the warps at 128 registers
-#endif
-#ifndef FV2D_FP64_FMINB
-#define FV2D_FP64_FMINB 4   // 4 x 128 threads at up to 128 registers
+#define FV2D_FP64_GMINB 6   // 6 x 128 threads at 80 registers: 400k-cell NS cylinder 2.75 ms per iteration, 2.81 with 8
+                            // (64 registers, spills), 2.79 with 5
 #endif
 template <bool SQUEEZE>
 __global__ void __launch_bounds__(FV2D_FP64_BLOCK, FV2D_FP64_GMINB)
-k_gradient(int nc, DevMesh<double> m, const Q4<double>* __restrict__ Q, const Q4<double>* __restrict__ Qprev,
-           const Q4<double>* __restrict__ Gprev, Q4<double>* __restrict__ Gout, Consts<double> k, int first_stage, int init_prims) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+k_gradient(int nc, DevMesh<double> m, const Q4<double>* Q, Q4<double>* Gout, Consts<double> k,
+           int first_stage, int init_prims) {
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
     if (c >= nc) return;
     const Fp fp;
-    gradient_cell<SQUEEZE, true>(c, fp, m, Q, Qprev, Gprev, Gout, k, first_stage, init_prims);
+    gradient_lane<SQUEEZE>(c, threadIdx.x & 3, fp, m, Q, Gout, k, first_stage, init_prims, Prior());
 }
+
+#ifndef FV2D_FP64_FMINB
+#define FV2D_FP64_FMINB 4   // 4 x 128 threads at up to 128 registers
+#endif
 
 // ------------------------------------------------------------------------------------------
 // Face kernel: reconstruction + boundary ghosts (reconstruction.cpp:22-80), NS face terms
@@ -493,18 +398,26 @@ k_gradient(int nc, DevMesh<double> m, const Q4<double>* __restrict__ Q, const Q4
 // (class_f.hpp:41-50, rusanov.cpp:20-36) and the face's residual contribution (res.cpp:81-89).
 // Writes t = (V*A) - (F*A) per face and, on the last stage of an iteration, the spectral term
 // (|Vn_avg| + c_avg)*A that the next time step sums (ssp_rk3.cpp:28-36).
+// First order: q + 0 dx + 0 dy is q, but for a -0 that meets a +0 product.
+__device__ __forceinline__ double first_order_state(double q, double dx, double dy) {
+    const bool pos = (__double2hiint(dx) & __double2hiint(dy)) >= 0;
+    return pos && __double_as_longlong(q) == (long long)0x8000000000000000ULL ? 0.0 : q;
+}
+
 // Powers of two travel through the formulas as exact scalings instead of operations: the average
 // state's sums S = L + R stand for 2 (L + R)/2, the wave speed t = |vn1 + vn2| + (c1 + c2) for 4 lambda,
 // the flux F2 for 2 F against half the area, the viscous flux V2 for 2 V (mu and k enter doubled), and
 // the remaining halves ride on multiply-adds.  Every rounded intermediate is the reference's times a
 // power of two, so the results are the same bits.  338 FP64 operations for an NS interior face.
-template <bool ORDER2, bool NS, bool LAST>
-__device__ __forceinline__ void face_flux(int f, const Fp& fp, const DevMesh<double>& m, const Q4<double>* __restrict__ Q,
-                                          const Q4<double>* __restrict__ G, Q4<double>* __restrict__ tout,
-                                          double* __restrict__ sout, const Consts<double>& k, int init_prims) {
+template <bool ORDER2, bool NS, bool LAST, class Wait>
+__device__ __forceinline__ void face_flux(int f, const Fp& fp, const DevMesh<double>& m, const Q4<double>* Q,
+                                          const Q4<double>* G, Q4<double>* tout, double* sout, const Consts<double>& k,
+                                          int init_prims, Wait wait) {
     const FaceGeo<double>& g = m.g;
     const int c1 = m.fc1[f], c2 = m.fc2[f];
     const double fnx = g.nx[f], fny = g.ny[f], A = g.area[f];
+    const double d1x = g.c1dx[f], d1y = g.c1dy[f], d2x = g.c2dx[f], d2y = g.c2dy[f];
+    wait();
     const Q4<double> q1 = ldq(Q, c1);
     Q4<double> g1x, g1y;
     if (ORDER2) { g1x = ldq(G, 2 * c1); g1y = ldq(G, 2 * c1 + 1); }
@@ -515,34 +428,17 @@ __device__ __forceinline__ void face_flux(int f, const Fp& fp, const DevMesh<dou
     Q4<double> g2x, g2y;
     if (ORDER2) { g2x = ldq(G, 2 * c2l); g2y = ldq(G, 2 * c2l + 1); }
     double L[4], Rq[4];
-    // first order: q + 0 dx + 0 dy is q, but for a -0 that meets a +0 product
-    auto first_order = [&](double q, double dx, double dy) {
-        const bool pos = (__double2hiint(dx) & __double2hiint(dy)) >= 0;
-        return pos && __double_as_longlong(q) == (long long)0x8000000000000000ULL ? 0.0 : q;
-    };
-    if (ORDER2) {
-        const double dx = g.c1dx[f], dy = g.c1dy[f];
 #pragma unroll
-        for (int j = 0; j < 4; j++) L[j] = fp.add(fp.add(q1.p[j], fp.mul(g1x.p[j], dx)), fp.mul(g1y.p[j], dy));
-    } else {
-        const double dx = g.c1dx[f], dy = g.c1dy[f];
-#pragma unroll
-        for (int j = 0; j < 4; j++) L[j] = first_order(q1.p[j], dx, dy);
-    }
+    for (int j = 0; j < 4; j++)
+        L[j] = ORDER2 ? fp.add(fp.add(q1.p[j], fp.mul(g1x.p[j], d1x)), fp.mul(g1y.p[j], d1y)) : first_order_state(q1.p[j], d1x, d1y);
     const double lrho = L[0];
     double lu, lv, lP;
     const Divisor ld = prims_r(L, k, fp, lu, lv, lP);
     const double lc = sqrt(k.gamma * ld.div(lP, fp));
     if (c2 >= 0) {
-        if (ORDER2) {
-            const double dx = g.c2dx[f], dy = g.c2dy[f];
 #pragma unroll
-            for (int j = 0; j < 4; j++) Rq[j] = fp.add(fp.add(q2.p[j], fp.mul(g2x.p[j], dx)), fp.mul(g2y.p[j], dy));
-        } else {
-            const double dx = g.c2dx[f], dy = g.c2dy[f];
-#pragma unroll
-            for (int j = 0; j < 4; j++) Rq[j] = first_order(q2.p[j], dx, dy);
-        }
+        for (int j = 0; j < 4; j++)
+            Rq[j] = ORDER2 ? fp.add(fp.add(q2.p[j], fp.mul(g2x.p[j], d2x)), fp.mul(g2y.p[j], d2y)) : first_order_state(q2.p[j], d2x, d2y);
     } else if (c2 == -1) {
 #pragma unroll
         for (int j = 0; j < 4; j++) Rq[j] = k.q_inf[j];
@@ -625,7 +521,6 @@ __device__ __forceinline__ void face_flux(int f, const Fp& fp, const DevMesh<dou
             Py = fp.mul(k.gm1, __fma_rn(fp.mul(S[0], fp.add(fp.mul(au, uy), fp.mul(av, vy))), -fp.half,
                                         __fma_rn(fp.mul(ry, ke), -fp.half, dQy[3])));
         } else if (c2 == -4) {
-            const double d1x = g.c1dx[f], d1y = g.c1dy[f];
             const double dn = fabs(sqrt(d1x * d1x + d1y * d1y));
             double cu, cv;
             if (init_prims) { cu = k.u_inf; cv = k.v_inf; }
@@ -668,12 +563,12 @@ __device__ __forceinline__ void face_flux(int f, const Fp& fp, const DevMesh<dou
 
 template <bool ORDER2, bool NS, bool LAST>
 __global__ void __launch_bounds__(FV2D_FP64_BLOCK, FV2D_FP64_FMINB)
-k_face(int nf, DevMesh<double> m, const Q4<double>* __restrict__ Q, const Q4<double>* __restrict__ G, Q4<double>* __restrict__ tout,
-       double* __restrict__ sout, Consts<double> k, int init_prims) {
+k_face(int nf, DevMesh<double> m, const Q4<double>* Q, const Q4<double>* G, Q4<double>* tout, double* sout, Consts<double> k,
+       int init_prims) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nf) return;
     const Fp fp;
-    face_flux<ORDER2, NS, LAST>(f, fp, m, Q, G, tout, sout, k, init_prims);
+    face_flux<ORDER2, NS, LAST>(f, fp, m, Q, G, tout, sout, k, init_prims, Prior());
 }
 
 // ------------------------------------------------------------------------------------------
@@ -735,7 +630,7 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
 constexpr int kUpdChunk = 4;   // incidences whose loads the residual gather issues together (4.6 % faster k_update)
 
 // S_c = sum of the face spectral terms in CSR order, loads issued a chunk at a time
-__device__ __forceinline__ double spectral_sum(const int* __restrict__ inc, const double* __restrict__ sface, int b, int e,
+__device__ __forceinline__ double spectral_sum(const int* __restrict__ inc, const double* sface, int b, int e,
                                                const Fp& fp) {
     double s = 0.0;
     constexpr int U = kUpdChunk;
@@ -743,7 +638,7 @@ __device__ __forceinline__ double spectral_sum(const int* __restrict__ inc, cons
         double v[U];
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (i0 + u < e) v[u] = sface[inc[i0 + u] >> 1];
+            if (i0 + u < e) v[u] = *(sface + (inc[i0 + u] >> 1));
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (i0 + u < e) s = fp.add(s, v[u]);
@@ -767,96 +662,290 @@ __device__ __forceinline__ bool positive<double>(double x) {
     return (unsigned long long)__double_as_longlong(x) - 1ull < 0x7ff0000000000000ull;
 }
 
-template <int STAGE>
-__device__ __forceinline__ double update_cell(int c, const Fp& fp, const DevMesh<double>& m, const Q4<double>* __restrict__ tface,
-                                              const double* __restrict__ sface, Q4<double>* __restrict__ Qn,
-                                              Q4<double>* __restrict__ Q1, Q4<double>* __restrict__ Q2, double* __restrict__ dt,
-                                              double* __restrict__ S, double smax, Q4<double>* __restrict__ Rout,
-                                              int* __restrict__ flag, const Consts<double>& k, int global_dt, double r[4]) {
-    const int* __restrict__ inc = m.inc;
-    double snext = 0.0;
+// What a cell's update reads of the mesh: its incidence range and first incidences, its volume.
+struct UpdateMesh {
+    int b = 0, e = 0, inc[kUpdChunk];
+    double vol = 1.0, rvol = 1.0;   // rvol: 1/vol, precomputed
+    __device__ __forceinline__ UpdateMesh(int c, const DevMesh<double>& m) {
+        b = m.inc_off[c];
+        e = m.inc_off[c + 1];
+        vol = m.vol[c];
+        rvol = m.rvol[c];
 #pragma unroll
-    for (int j = 0; j < 4; j++) r[j] = 0.0;
-    const int b = m.inc_off[c], e = m.inc_off[c + 1];
+        for (int u = 0; u < kUpdChunk; u++) inc[u] = b + u < e ? m.inc[b + u] : 0;
+    }
+};
+
+// One component j of cell c's update; returns its residual component.
+template <int STAGE>
+__device__ __forceinline__ double update_lane(int c, int j, const Fp& fp, const DevMesh<double>& m, const UpdateMesh& um,
+                                              const Q4<double>* tface, Q4<double>* Qn, Q4<double>* Q1, Q4<double>* Q2,
+                                              double dtc, Q4<double>* Rout, int* flag) {
+    const double* t = reinterpret_cast<const double*>(tface);
+    const size_t o = 4 * (size_t)c + j;
+    const int b = um.b, e = um.e;
+    const double qn = reinterpret_cast<const double*>(Qn)[o];
+    const double qs = STAGE == 0 ? 0.0 : reinterpret_cast<const double*>(STAGE == 1 ? Q1 : Q2)[o];
+    double r = 0.0;
     // chunks of kUpdChunk incidences: every record and face contribution of a chunk is requested
     // before the first is summed (more loads in flight per thread); the sums keep CSR order
     constexpr int U = kUpdChunk;
     for (int i0 = b; i0 < e; i0 += U) {
         int iv[U];
-        Q4<double> tv[U];
+        double tv[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) iv[u] = i0 == b ? um.inc[u] : i0 + u < e ? m.inc[i0 + u] : 0;
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (i0 + u < e) iv[u] = inc[i0 + u];
+            if (i0 + u < e) tv[u] = t[4 * (size_t)(iv[u] >> 1) + j];
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (i0 + u < e) tv[u] = ldq(tface, iv[u] >> 1);
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (i0 + u < e) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) r[j] = fp.add(r[j], neg_if(tv[u].p[j], iv[u] & 1));   // side 1: r -= t
-            }
-        }
+            if (i0 + u < e) r = fp.add(r, neg_if(tv[u], iv[u] & 1));   // side 1: r -= t
     }
-    const double vc = m.vol[c];
-    const Divisor vd(vc, m.rvol[c], fp);   // 1/vol precomputed
-#pragma unroll
-    for (int j = 0; j < 4; j++) r[j] = vd.div(r[j], fp);
-    if (Rout) { Q4<double> rr; for (int j = 0; j < 4; j++) rr.p[j] = r[j]; Rout[c] = rr; }
-    const Q4<double> qn = ldq(Qn, c);
-    Q4<double> out;
-    double dtc;
-    if (STAGE == 0) {
-        dtc = (k.two_cfl * vc) / (global_dt ? smax : S[c]);
-        dt[c] = dtc;
-    } else {
-        dtc = dt[c];
+    {   // r / vol: two residual corrections from RN(r*y), as Recip (Divisor's digits would cost every lane more)
+        const double q0 = fp.mul(r, um.rvol), q1 = __fma_rn(__fma_rn(-um.vol, q0, r), um.rvol, q0);
+        r = (__double_as_longlong(r) << 1) == 0 ? q0 : __fma_rn(__fma_rn(-um.vol, q1, r), um.rvol, q1);
     }
+    if (Rout) reinterpret_cast<double*>(Rout)[o] = r;
+    const double dr = fp.mul(dtc, r);
+    double out;
     if (STAGE == 0) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) out.p[j] = fp.add(qn.p[j], fp.mul(dtc, r[j]));
-        Q1[c] = out;
+        out = fp.add(qn, dr);
+        reinterpret_cast<double*>(Q1)[o] = out;
     } else if (STAGE == 1) {   // 3/4 Qn + 1/4 Q1 + 1/4 dt R, the exact quarters on the multiply-adds
-        const Q4<double> q1 = ldq(Q1, c);
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            out.p[j] = __fma_rn(fp.mul(dtc, r[j]), 0.25, __fma_rn(q1.p[j], 0.25, fp.mul(0.75, qn.p[j])));
-        Q2[c] = out;
+        out = __fma_rn(dr, 0.25, __fma_rn(qs, 0.25, fp.mul(0.75, qn)));
+        reinterpret_cast<double*>(Q2)[o] = out;
     } else {
-        const Q4<double> q2 = ldq(Q2, c);
-        const double dt23 = fp.mul(2.0 / 3.0, dtc);
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            out.p[j] = fp.add(fp.add(fp.mul(1.0 / 3.0, qn.p[j]), fp.mul(2.0 / 3.0, q2.p[j])), fp.mul(dt23, r[j]));
-        Qn[c] = out;
-        snext = spectral_sum(inc, sface, b, e, fp);
-        S[c] = snext;
+        out = fp.add(fp.add(fp.mul(1.0 / 3.0, qn), fp.mul(2.0 / 3.0, qs)), fp.mul(fp.mul(2.0 / 3.0, dtc), r));
+        reinterpret_cast<double*>(Qn)[o] = out;
     }
-    if (!positive(out.p[0]) || !positive(out.p[3])) atomicOr(flag, 1);
-    return snext;
+    if ((j == 0 || j == 3) && !positive(out)) atomicOr(flag, 1);
+    return r;
 }
 
-#ifndef FV2D_UPD_BLOCK
-#define FV2D_UPD_BLOCK 256   // threads per block of the single-solve update kernel
-#endif
+// Threads per block of the update kernel: four lanes (one component each) per cell; the block's first
+// warp also holds one lane per cell for what a cell needs once: its time step in the first stage
+// (one division) and its spectral sum in the last.  The second stage, which does not read it, zeroes
+// the spectral maximum that the last accumulates.
+constexpr int kUpdBlock = 128, kUpdCells = kUpdBlock / 4;
+
 template <int STAGE>
-__global__ void __launch_bounds__(FV2D_UPD_BLOCK)
-k_update(int nc, DevMesh<double> m, const Q4<double>* __restrict__ tface, const double* __restrict__ sface,
-         Q4<double>* __restrict__ Qn, Q4<double>* __restrict__ Q1, Q4<double>* __restrict__ Q2, double* __restrict__ dt,
-         double* __restrict__ S, double* __restrict__ smax, Q4<double>* __restrict__ Rout, int* __restrict__ flag,
-         Consts<double> k, int global_dt) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    double snext = 0.0;
-    if (c < nc) {
-        const Fp fp;
-        double r[4];
-        snext = update_cell<STAGE>(c, fp, m, tface, sface, Qn, Q1, Q2, dt, S, (STAGE == 0 && global_dt) ? *smax : 0.0, Rout, flag,
-                                   k, global_dt, r);
+__global__ void __launch_bounds__(kUpdBlock)
+k_update(int nc, DevMesh<double> m, const Q4<double>* tface, const double* sface, Q4<double>* Qn,
+         Q4<double>* Q1, Q4<double>* Q2, double* dt, double* S, double* smax, Q4<double>* Rout, int* flag, Consts<double> k,
+         int global_dt) {
+    __shared__ double sdt[kUpdCells];
+    const Fp fp;
+    const int c0 = blockIdx.x * kUpdCells, c = c0 + (threadIdx.x >> 2), j = threadIdx.x & 3, cw = c0 + threadIdx.x;
+    const UpdateMesh um(min(c, nc - 1), m);
+    Prior()();
+    if (STAGE == 0) {
+        if (threadIdx.x < kUpdCells && cw < nc) {
+            const double d = (k.two_cfl * m.vol[cw]) / (global_dt ? *smax : S[cw]);
+            sdt[threadIdx.x] = d;
+            dt[cw] = d;
+        }
+        __syncthreads();
     }
-    if (STAGE == 2) {
-        const double mx = block_max(c < nc ? snext : 0.0);
-        if (threadIdx.x == 0) atomic_max_pos(smax, mx);
+    if (STAGE == 1 && blockIdx.x == 0 && threadIdx.x == 0) *smax = 0.0;
+    if (c < nc)
+        update_lane<STAGE>(c, j, fp, m, um, tface, Qn, Q1, Q2, STAGE == 0 ? sdt[threadIdx.x >> 2] : dt[c], Rout, flag);
+    if (STAGE == 2 && threadIdx.x < kUpdCells) {
+        double s = 0.0;
+        if (cw < nc) {
+            s = spectral_sum(m.inc, sface, m.inc_off[cw], m.inc_off[cw + 1], fp);
+            S[cw] = s;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s = max2(s, __shfl_xor_sync(0xffffffffu, s, o));
+        if (threadIdx.x == 0) atomic_max_pos(smax, s);
     }
+}
+
+// Two lanes per face, for meshes small enough that every warp has its SM quarter's FP64 pipe to itself, so
+// that the length of a lane's chain of operations is the pass's time: lane h = 0 takes cell c1's side, components 0
+// and 1 of the flux and the x derivatives, lane h = 1 cell c2's side, components 2 and 3 and the y
+// derivatives.  Every value is computed by the expression face_flux uses, so the bits are the same;
+// about 205 operations a lane for an NS interior face against 352.  All 32 lanes call (act: the lane
+// pair has a face).  (With programmatic launches: 512 Euler quads 58 -> 50 us per iteration, 2k NS
+// polygons 80 -> 72; with two warps to a quarter the extra work loses, 8k NS polygons 118 -> 131.)
+template <bool ORDER2, bool NS>
+__device__ __forceinline__ void face_pair(int f, int h, bool act, const Fp& fp, const DevMesh<double>& m, const Q4<double>* Q,
+                                          const Q4<double>* G, Q4<double>* tout, double* sout, const Consts<double>& k,
+                                          int init_prims, bool last, Prior wait) {
+    constexpr unsigned FULL = 0xffffffffu;
+    auto other = [&](double x) { return __shfl_xor_sync(FULL, x, 1); };
+    // the partner's value of this lane's components: send the partner's pair, keep one's own
+    auto swap2 = [&](const double v[4], double& a, double& b) {
+        a = other(h ? v[0] : v[2]);
+        b = other(h ? v[1] : v[3]);
+    };
+    const FaceGeo<double>& g = m.g;
+    const int ff = act ? f : 0;
+    const int c1 = m.fc1[ff], c2 = m.fc2[ff];
+    const bool inner = c2 >= 0;
+    const int cell = h && inner ? c2 : c1;
+    const double fnx = g.nx[ff], fny = g.ny[ff];
+    const double dx = h ? g.c2dx[ff] : g.c1dx[ff], dy = h ? g.c2dy[ff] : g.c1dy[ff];
+    const double A = g.area[ff];
+    wait();
+    const Q4<double> q = Q[cell];
+    Q4<double> gx, gy;
+    if (ORDER2) { gx = G[2 * (size_t)cell]; gy = G[2 * (size_t)cell + 1]; }
+    double X[4];   // this side's face state
+    if (ORDER2) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) X[j] = fp.add(fp.add(q.p[j], fp.mul(gx.p[j], dx)), fp.mul(gy.p[j], dy));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) X[j] = first_order_state(q.p[j], dx, dy);
+    }
+    double u = 0.0, v = 0.0, P = 0.0, c = 0.0;
+    auto side = [&] {
+        const Divisor r = prims_r(X, k, fp, u, v, P);
+        c = sqrt(k.gamma * r.div(P, fp));
+    };
+    if (!h || inner) side();
+    if (__any_sync(FULL, !inner)) {   // boundary faces: lane 1's state is a ghost of lane 0's
+        double L[4], lu, lv, lP;
+#pragma unroll
+        for (int j = 0; j < 4; j++) L[j] = other(X[j]);
+        lu = other(u);
+        lv = other(v);
+        lP = other(P);
+        if (h && !inner) {
+            if (c2 == -1) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) X[j] = k.q_inf[j];
+            } else if (c2 == -2) {
+                const double vn = lu * fnx + lv * fny;
+                cons(L[0], lu - 2.0 * vn * fnx, lv - 2.0 * vn * fny, lP, k, X);
+            } else if (c2 == -3) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) X[j] = L[j];
+            } else {
+                cons(L[0], -lu, -lv, lP, k, X);
+            }
+            side();
+        }
+    }
+    if (m.fval && act && (!h || inner)) {
+        Q4<double> o;
+#pragma unroll
+        for (int j = 0; j < 4; j++) o.p[j] = X[j];
+        m.fval[2 * (size_t)f + h] = o;
+    }
+    const double vn = fp.add(fp.mul(u, fnx), fp.mul(v, fny));
+    const double t4 = fp.add(fabs(fp.add(vn, other(vn))), fp.add(c, other(c)));
+    const double Ah = fp.mul(A, fp.half);
+    // this lane's two components: states of both sides, 2 F
+    double oX[2], F2[2];
+    swap2(X, oX[0], oX[1]);
+    const double myX[2] = {h ? X[2] : X[0], h ? X[3] : X[1]};
+    {
+        const double F[4] = {fp.mul(X[0], vn), fp.add(fp.mul(fp.mul(X[0], u), vn), fp.mul(P, fnx)),
+                             fp.add(fp.mul(fp.mul(X[0], v), vn), fp.mul(P, fny)), fp.mul(vn, fp.add(X[3], P))};
+        double oF[2];
+        swap2(F, oF[0], oF[1]);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const double d = h ? fp.sub(myX[i], oX[i]) : fp.sub(oX[i], myX[i]);   // R - L
+            F2[i] = k.roe ? -202.0 : __fma_rn(fp.mul(t4, d), -fp.half, fp.add(h ? F[2 + i] : F[i], oF[i]));
+        }
+    }
+    double V2[2] = {0.0, 0.0};
+    if (NS && ORDER2) {
+        double S[4];   // twice the average state
+        {
+            const double a = fp.add(myX[0], oX[0]), b = fp.add(myX[1], oX[1]), oa = other(a), ob = other(b);
+            S[0] = h ? oa : a; S[1] = h ? ob : b; S[2] = h ? a : oa; S[3] = h ? b : ob;
+        }
+        const Divisor sd(S[0], fp);
+        const double mine = sd.div(h ? S[2] : S[1], fp), theirs = other(mine);
+        const double au = h ? theirs : mine, av = h ? mine : theirs;
+        const double ke = fp.add(fp.mul(au, au), fp.mul(av, av));
+        const double aP2 = fp.mul(__fma_rn(fp.mul(S[0], ke), -fp.half, S[3]), k.gm1);   // twice the pressure
+        const double nh = h ? fny : fnx;
+        double U = 0.0, V = 0.0, dP = 0.0, r = 0.0;   // this direction's derivatives of u, v, P, rho
+        {
+            // differences and tangential derivatives of this lane's components, then of all four
+            double oq[2], ogx[2], ogy[2], dl[4], dm2[4];
+            swap2(q.p, oq[0], oq[1]);
+            swap2(gx.p, ogx[0], ogx[1]);
+            swap2(gy.p, ogy[0], ogy[1]);
+            const Divisor dd(inner ? fabs(g.dist[ff]) : 1.0, inner ? m.rdist[ff] : 1.0, fp);
+            const double mxf = -fny, myf = fnx, lh = inner ? (h ? g.ly[ff] : g.lx[ff]) : 0.0;
+            double a[2], b[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const double mq = h ? q.p[2 + i] : q.p[i], mgx = h ? gx.p[2 + i] : gx.p[i], mgy = h ? gy.p[2 + i] : gy.p[i];
+                const double q1 = h ? oq[i] : mq, q2 = h ? mq : oq[i], g1x = h ? ogx[i] : mgx, g1y = h ? ogy[i] : mgy,
+                             g2x = h ? mgx : ogx[i], g2y = h ? mgy : ogy[i];
+                a[i] = dd.div(fp.sub(q2, q1), fp);
+                b[i] = fp.add(fp.add(fp.add(fp.mul(g1x, mxf), fp.mul(g1y, myf)), fp.mul(g2x, mxf)), fp.mul(g2y, myf));
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const double oa = other(a[i]), ob = other(b[i]);
+                dl[i] = h ? oa : a[i]; dl[2 + i] = h ? a[i] : oa;
+                dm2[i] = h ? ob : b[i]; dm2[2 + i] = h ? b[i] : ob;
+            }
+            if (inner) {
+                double dQ[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) dQ[j] = __fma_rn(fp.mul(dm2[j], lh), fp.half, fp.mul(dl[j], lh));
+                r = dQ[0];
+                U = __fma_rn(sd.div(fp.mul(r, au), fp), -2.0, dQ[1]);
+                V = __fma_rn(sd.div(fp.mul(r, h ? au : av), fp), -2.0, dQ[2]);   // reconstruction.cpp:155 uses u for y
+                dP = fp.mul(k.gm1, __fma_rn(fp.mul(S[0], fp.add(fp.mul(au, U), fp.mul(av, V))), -fp.half,
+                                            __fma_rn(fp.mul(r, ke), -fp.half, dQ[3])));
+            } else if (c2 == -4) {
+                const double d1x = g.c1dx[ff], d1y = g.c1dy[ff];
+                const double dn = fabs(sqrt(d1x * d1x + d1y * d1y));
+                double cu, cv;
+                if (init_prims) { cu = k.u_inf; cv = k.v_inf; }
+                else { cu = q.p[1] / q.p[0]; cv = q.p[2] / q.p[0]; }   // both lanes hold cell c1's state here
+                const Divisor nd(dn, fp);
+                U = nd.div(-cu, fp) * nh;
+                V = nd.div(-cv, fp) * nh;
+            }
+        }
+        const double oU = other(U), oV = other(V);
+        const double ux = h ? oU : U, vx = h ? oV : V, uy = h ? U : oU, vy = h ? V : oV;
+        double ta = 0.0, tb = 0.0, dT = 0.0;   // row h of twice the stress tensor; half this direction's dT
+        if (c2 != -2) {   // SLIP_WALL with NS: tau and grad T keep their initial zeros (:104-106)
+            const double third = div3(fp.add(ux, vy));
+            const double diag = fp.mul(4.0 * k.mu, fp.sub(h ? vy : ux, third)), off = fp.mul(2.0 * k.mu, fp.add(uy, vx));
+            ta = h ? off : diag;
+            tb = h ? diag : off;
+            const double den = fp.mul(fp.mul(k.R, S[0]), S[0]);   // 4 R rho^2
+            dT = Recip<double>::div(fp.sub(fp.mul(dP, S[0]), fp.mul(r, aP2)), den, __drcp_rn(den));
+        }
+        const double row = fp.add(fp.mul(ta, fnx), fp.mul(tb, fny));
+        const double heat = fp.mul(nh, fp.add(fp.add(fp.mul(au, ta), fp.mul(av, tb)), fp.mul(4.0 * k.k, dT)));
+        const double oheat = other(heat);
+        V2[0] = h ? row : 0.0;
+        V2[1] = h ? fp.add(oheat, heat) : row;
+    }
+    if (!act) return;
+    double t[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        if (!(NS && ORDER2)) t[i] = zero_minus(fp.mul(F2[i], Ah));
+        else t[i] = !h && i == 0 ? zero_minus(fp.mul(F2[i], Ah)) : fp.sub(fp.mul(V2[i], Ah), fp.mul(F2[i], Ah));
+    }
+    *reinterpret_cast<double2*>(reinterpret_cast<double*>(tout + f) + 2 * h) = make_double2(t[0], t[1]);
+    if (last && !h) sout[f] = k.roe ? (fabs(k.vn0) + k.c0) * A : fp.mul(t4, Ah);
+}
+
+template <bool ORDER2, bool NS, bool LAST>
+__global__ void __launch_bounds__(FV2D_FP64_BLOCK, FV2D_FP64_FMINB)
+k_face_pair(int nf, DevMesh<double> m, const Q4<double>* Q, const Q4<double>* G, Q4<double>* tout, double* sout, Consts<double> k,
+            int init_prims) {
+    const int f = (blockIdx.x * blockDim.x + threadIdx.x) >> 1;
+    if ((f & ~15) >= nf) return;   // whole warps
+    const Fp fp;
+    face_pair<ORDER2, NS>(f, threadIdx.x & 1, f < nf, fp, m, Q, G, tout, sout, k, init_prims, LAST, Prior());
 }
 
 // Geometry-only reciprocals of a mesh (or of one solve's ranges in a batch arena): rdist = 1/|dist|

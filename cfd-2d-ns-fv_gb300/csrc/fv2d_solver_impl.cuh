@@ -42,6 +42,10 @@ public:
         DeviceLayout L;
         build_layout(m, L);
         nc_ = m.nc; nf_ = m.nf; ninc_ = L.ninc;
+        int dev = 0, sms = 1;
+        FV2D_CUDA(cudaGetDevice(&dev));
+        FV2D_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        small_ = nf_ <= 64LL * sms;
         order2_ = cs.order == 2;
         ns_ = cs.eqn == FV2D_NS;
         squeeze_ = cs.limiter == FV2D_LIM_SQUEEZE;
@@ -199,29 +203,17 @@ public:
     int stage() override {
         const int s = stage_;
         Q4<T>* qin = Q_[s];
-        const int p = (s + 2) % 3;
         if (order2_) {
-            constexpr int B = FV2D_FP64_BLOCK;
-            launch(K_GRADIENT, nc_, [&](int gr) {
-                if (squeeze_)
-                    k_gradient<true><<<gr, B, 0, stream_>>>(nc_, dm_, qin, Q_[p], G_[p], G_[s], k_, fresh_ ? 1 : 0,
-                                                              init_prims_ ? 1 : 0);
-                else
-                    k_gradient<false><<<gr, B, 0, stream_>>>(nc_, dm_, qin, Q_[p], G_[p], G_[s], k_, fresh_ ? 1 : 0,
-                                                               init_prims_ ? 1 : 0);
-            }, B);
+            auto* kg = squeeze_ ? k_gradient<true> : k_gradient<false>;
+            FV2D_CUDA(launch(K_GRADIENT, kg, 4LL * nc_, FV2D_FP64_BLOCK, nc_, dm_, (const Q4<T>*)qin, G_[s], k_, fresh_ ? 1 : 0, init_prims_ ? 1 : 0));
         }
-        launch(K_FACE, nf_, [&](int gr) { launch_face(gr, qin, G_[s], s == 2); }, FV2D_FP64_BLOCK);
-        if (s == 2) FV2D_CUDA(cudaMemsetAsync(smax_, 0, sizeof(T), stream_));
+        const bool pair = small_;
+        FV2D_CUDA(launch(K_FACE, face_kernel(pair, s == 2), pair ? 2LL * nf_ : nf_, FV2D_FP64_BLOCK, nf_, dm_, (const Q4<T>*)qin,
+                         (const Q4<T>*)G_[s], t_, s_, k_, init_prims_ ? 1 : 0));
         Q4<T>* rout = (store_every_ || s == 2) ? R_ : nullptr;
-        launch(K_UPDATE, nc_, [&](int gr) {
-            if (s == 0)
-                k_update<0><<<gr, FV2D_UPD_BLOCK, 0, stream_>>>(nc_, dm_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout, flag_, k_, global_dt_);
-            else if (s == 1)
-                k_update<1><<<gr, FV2D_UPD_BLOCK, 0, stream_>>>(nc_, dm_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout, flag_, k_, global_dt_);
-            else
-                k_update<2><<<gr, FV2D_UPD_BLOCK, 0, stream_>>>(nc_, dm_, t_, s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout, flag_, k_, global_dt_);
-        }, FV2D_UPD_BLOCK);
+        auto* ku = s == 0 ? k_update<0> : s == 1 ? k_update<1> : k_update<2>;
+        FV2D_CUDA(launch(K_UPDATE, ku, 4LL * nc_, kUpdBlock, nc_, dm_, (const Q4<T>*)t_, (const T*)s_, Q_[0], Q_[1], Q_[2], dt_, S_, smax_, rout,
+                         flag_, k_, global_dt_));
         FV2D_CUDA(cudaGetLastError());
         if (s == 0) { fresh_ = false; init_prims_ = false; }
         last_stage_ = s;
@@ -350,16 +342,34 @@ public:
     long long device_bytes() const override { return (long long)arena_bytes_; }
 
 private:
-    void launch_face(int gr, const Q4<T>* qin, const Q4<T>* G, bool last) {
-#define FV2D_FACE(O2, NS, LAST) \
-    k_face<O2, NS, LAST><<<gr, FV2D_FP64_BLOCK, 0, stream_>>>(nf_, dm_, qin, G, t_, s_, k_, init_prims_ ? 1 : 0)
-        if (order2_) {
-            if (ns_) { if (last) FV2D_FACE(true, true, true); else FV2D_FACE(true, true, false); }
-            else { if (last) FV2D_FACE(true, false, true); else FV2D_FACE(true, false, false); }
-        } else {
-            if (last) FV2D_FACE(false, false, true); else FV2D_FACE(false, false, false);
-        }
-#undef FV2D_FACE
+    using FaceKernel = void (*)(int, DevMesh<T>, const Q4<T>*, const Q4<T>*, Q4<T>*, T*, Consts<T>, int);
+    FaceKernel face_kernel(bool pair, bool last) const {
+        if (!order2_) return pair ? (last ? k_face_pair<false, false, true> : k_face_pair<false, false, false>)
+                                  : (last ? k_face<false, false, true> : k_face<false, false, false>);
+        if (ns_) return pair ? (last ? k_face_pair<true, true, true> : k_face_pair<true, true, false>)
+                             : (last ? k_face<true, true, true> : k_face<true, true, false>);
+        return pair ? (last ? k_face_pair<true, false, true> : k_face_pair<true, false, false>)
+                    : (last ? k_face<true, false, true> : k_face<true, false, false>);
+    }
+
+    // A stage kernel over n threads; of a small solve as a programmatic dependent of the kernel before it
+    // in the stream (its CTAs are placed while that one runs and wait for its results themselves: 58 ->
+    // 54 us per iteration of 512 quads).  Not of larger ones, whose next CTAs would be placed where the
+    // running kernel leaves room instead of evenly (24k quads 111 -> 178 us).
+    template <class... KA, class... A>
+    cudaError_t launch(int kid, void (*kernel)(KA...), long long n, int block, A... args) {
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)std::max<long long>(1, (n + block - 1) / block));
+        cfg.blockDim = dim3((unsigned)block);
+        cfg.stream = stream_;
+        cfg.attrs = &at;
+        cfg.numAttrs = small_ && !timing_ ? 1 : 0;
+        cudaError_t e = cudaSuccess;
+        launch(kid, 1, [&](int) { e = cudaLaunchKernelEx(&cfg, kernel, KA(args)...); });
+        return e;
     }
 
     template <class F>
@@ -393,6 +403,7 @@ private:
     int global_dt_ = 0;
     bool fresh_ = true, init_prims_ = true, store_every_ = false, graphs_ = true, timing_ = false;
     bool graph_store_every_ = false;
+    bool small_ = false;   // two lanes per face are at most one warp per SM quarter (16 faces x 4 quarters per SM)
     int last_stage_ = -1;
     cudaStream_t stream_ = nullptr;
     cudaGraphExec_t graph_exec_ = nullptr;
