@@ -42,14 +42,15 @@ def _units():
         ("fv2d_output.cpp", host),
         ("fv2d_api.cu", [nvcc] + common),
         # the FP64 engine must not contract a*b+c: bit-identical with the reference
-        ("fv2d_fp64.cu", [nvcc] + common + ["-fmad=false"]),
+        # (on the host too: the freestream state is evaluated there, and Arm compilers contract by default)
+        ("fv2d_fp64.cu", [nvcc] + common + ["-fmad=false", "-Xcompiler", "-ffp-contract=off"]),
         # the FP32 engine: a single solve and a batch run the same fused stage kernels, so FMA
         # contraction is allowed (both round alike); divisions and square roots use the
         # approximate (few-ulp) forms
         # FP32 engine: approximate division and square root, denormals flushed to zero (the flow's
         # FP32 values are far above FP32's normal range; norms are summed in FP64)
         ("fv2d_tiled.cu", [nvcc] + common + ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]),
-        ("fv2d_noalloc.cu", [nvcc] + common + ["-fmad=false"]),
+        ("fv2d_noalloc.cu", [nvcc] + common + ["-fmad=false", "-Xcompiler", "-ffp-contract=off"]),
     ]
 
 

@@ -233,15 +233,16 @@ void* fv2d_batch_stream(fv2d_batch* b);
  * solution_poly_order = 0, src/solver/res.cpp:21: boundary ghosts, Rusanov flux, gather / volume;
  * no viscous flux, as in the reference at first order) and allocates nothing.
  *
- * Its per-face scratch is a static device array of FV2D_NOALLOC_MAX_FACES x 4 doubles (8 MiB)
- * that lives with the library's device code on each GPU until the process exits; meshes with more
+ * Its scratch is two static device arrays, FV2D_NOALLOC_MAX_FACES x 4 doubles per face (8 MiB) and the
+ * primitives of as many cells as such a mesh can have (5.3 MiB), that live with the library's
+ * device code on each GPU until the process exits; meshes with more
  * faces are rejected with FV2D_ERR_ARG (use fv2d_create / fv2d_stage for those).  The first call on
- * each device looks up that array's device address with the device current; make that first call
+ * each device looks up the arrays' device addresses with the device current; make that first call
  * before any stream capture.  Under CUDA's lazy module loading (the default; CUDA_MODULE_LOADING
- * unset or LAZY) the library's device code and this array are only placed on a device by that first
+ * unset or LAZY) the library's device code and these arrays are only placed on a device by that first
  * call, so the FIRST call does take device memory: a host whose allocator reserves the GPU's memory
  * makes one warm-up call per device (any small mesh) before it reserves its pool, or runs with
- * CUDA_MODULE_LOADING=EAGER.  Every later call allocates nothing.  The looked-up address belongs to
+ * CUDA_MODULE_LOADING=EAGER.  Every later call allocates nothing.  The looked-up addresses belong to
  * the device's primary context: resetting the device (cudaDeviceReset) after the first call is not
  * supported in the same process.  The scratch is fully rewritten before it is read, so no state
  * carries over between calls, but all calls share it: calls that overlap on the GPU (other
