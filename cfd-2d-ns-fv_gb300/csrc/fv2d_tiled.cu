@@ -207,6 +207,9 @@ public:
         FV2D_T(cudaFuncSetAttribute(k_tstage<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmTotal));
         FV2D_T(cudaFuncSetAttribute(k_tstage<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmTotal));
         FV2D_T(cudaFuncSetAttribute(k_tstage<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmTotal));
+        // the limit, not a plan's own size: the attribute is the function's, shared by every handle
+        FV2D_T(cudaFuncSetAttribute(k_titer<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmTotalMax));
+        FV2D_T(cudaFuncSetAttribute(k_titer<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmTotalMax));
         int per = 0;
         FV2D_T(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tstage<1>, kTileCore, kSmTotal));
         grid_ = std::max(1, per) * sms_;
@@ -240,7 +243,6 @@ public:
         for (const void* f : {(const void*)k_titer<2>, (const void*)k_titer<3>}) {
             int per = 0;
             if (off > kSmTotalMax) continue;
-            FV2D_T(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, off));
             FV2D_T(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kTileCore, off));
             if (hi_tiles_ <= (long long)per * sms_) { iter_fn_ = f; break; }
         }

@@ -102,3 +102,20 @@ def test_batch_with_removed_solves(pkg):
         assert bits_equal(b.get_state(ids[i]), s.get_state())
         s.close()
     b.close()
+
+
+def test_handles_of_different_plans_in_turn(pkg):
+    """A handle with larger tiles steps after one with smaller tiles was planned (and the other way
+    round): each handle's launches have its own shared-memory size."""
+    big = pkg.meshgen.voronoi_bump_channel(76000, seed=3)
+    small = pkg.meshgen.channel_bump_quads(13, 5)
+    case = case_of(pkg, eqn="EULER")
+    a, b = (pkg.Solver(g, case, precision=pkg.FP32) for g in (big, small))
+    for s in (a, b, a, b):
+        s.step(1)
+    for s, g in ((a, big), (b, small)):
+        t = pkg.Solver(g, case, precision=pkg.FP32)
+        t.stage(6)
+        assert bits_equal(s.get_state(), t.get_state())
+        t.close()
+        s.close()
