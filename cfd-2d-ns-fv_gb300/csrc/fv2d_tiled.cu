@@ -385,9 +385,23 @@ public:
         // (the stage's tile counter was zeroed by the previous stage's kernel; the GLOBAL-dt maxima
         // by the second stage's)
         timed(st, [&] {
-            // persistent grid (CTAs that take tiles until none is left) or one CTA per tile slot
-            const int gr = full_grid_ ? (int)std::max<long long>(1, hi_tiles_) : grid_;
-            if (st == 0) k_tstage<0><<<gr, kTileCore, kSmTotal, stream_>>>(A_);
+            // persistent grid (CTAs that take tiles until none is left) or one CTA per tile slot (always
+            // of the first-order kernel)
+            const int gr = full_grid_ || first_ ? (int)std::max<long long>(1, hi_tiles_) : grid_;
+            if (first_) {
+                TFirst f = first_plan_;
+                cudaLaunchConfig_t cfg = {};
+                cfg.gridDim = dim3((unsigned)gr);
+                cfg.blockDim = dim3(kTileCore);
+                cfg.dynamicSmemBytes = (size_t)first_smem(f.flux, f.grad);
+                cfg.stream = stream_;
+                cudaLaunchAttribute at;
+                at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+                at.val.programmaticStreamSerializationAllowed = 1;
+                cfg.attrs = &at;
+                cfg.numAttrs = 1;
+                cudaLaunchKernelEx(&cfg, st == 0 ? k_tfirst<0> : st == 1 ? k_tfirst<1> : k_tfirst<2>, A_, f);
+            } else if (st == 0) k_tstage<0><<<gr, kTileCore, kSmTotal, stream_>>>(A_);
             else if (st == 1) k_tstage<1><<<gr, kTileCore, kSmTotal, stream_>>>(A_);
             else k_tstage<2><<<gr, kTileCore, kSmTotal, stream_>>>(A_);
         });
@@ -560,7 +574,19 @@ private:
             if (solves_[k].active) hi = std::max<long long>(hi, (long long)solves_[k].first_tile + solves_[k].ntiles);
         *cnt_pin_ = (int)hi;
         iter_planned_ = false;
-        if (full_grid_ && hi != hi_tiles_) drop_graphs();
+        // first-order kernels where no active solve needs gradients, planned for the largest tile
+        bool first = hi > 0;
+        TFirst f{};
+        for (int k = 0; k < caps_.solves; k++) {
+            if (!solves_[k].active) continue;
+            first = first && !pin_params_[k].order2;
+            f.flux = std::max(f.flux, (solves_[k].image->max_flux + 3) & ~3);
+            f.grad = std::max(f.grad, solves_[k].image->max_grad);
+        }
+        if (first != first_ || (first && (f.flux != first_plan_.flux || f.grad != first_plan_.grad))) drop_graphs();
+        first_ = first;
+        first_plan_ = f;
+        if ((full_grid_ || first_) && hi != hi_tiles_) drop_graphs();
         hi_tiles_ = hi;
         if (s.ntiles)
             FV2D_T(cudaMemcpyAsync((void*)(A_.tiles + s.first_tile), d, sizeof(TileDesc) * (size_t)s.ntiles,
@@ -590,6 +616,8 @@ private:
     struct Pending { int kid; cudaEvent_t a, b; };
 
     TIter iter_{};                       // the whole-iteration kernel's plan for the active solves
+    bool first_ = false;                 // every active solve is first order: k_tfirst's stages
+    TFirst first_plan_{};
     const void* iter_fn_ = nullptr;      // its variant, null: the tiles do not all fit at once
     int iter_smem_ = 0;
     bool iter_planned_ = false;

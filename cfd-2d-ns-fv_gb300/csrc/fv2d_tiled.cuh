@@ -18,8 +18,8 @@
 // A face shared by two tiles is evaluated by both, with the same inputs and the same code, so both
 // get the same value; every per-cell sum runs in a fixed order, so results do not depend on the
 // tile schedule, and a solve gives the same bits alone and in a batch (both run these kernels).
-// Solves whose tiles all fit on the GPU at once run whole iterations in one launch (k_titer, the same
-// passes).
+// First-order solves have a smaller kernel per stage (k_tfirst); solves whose tiles all fit on the GPU at once
+// run whole iterations in one launch (k_titer).  Both run the same passes.
 #pragma once
 
 #include <cstdint>
@@ -170,6 +170,9 @@ struct TileView {
                                       // (1M-cell NS cylinder 309.6 -> 304.0 us per iteration)
 };
 
+// Of a programmatic dependent launch: all writes of the kernels before are visible after it.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // The limited LSQ gradient of one core or ring-1 cell (local slot gI).  ghost(r): the state of the
 // cell that a no-slip face's gradient ghost reads; prev(): the cell's previous-stage state.
 template <class Ghost, class Prev>
@@ -286,7 +289,7 @@ __device__ __forceinline__ void tile_gradient(const TileView& v, const Consts<fl
 // stage, its spectral term to w_sp[r].  (w_t and w_sp may be the record's own displacement and
 // normal-x rows: both are read before they are written.)  INTERIOR: the record joins two cells, so
 // the boundary branches go and both sides' reconstructions can be scheduled together.
-template <bool INTERIOR>
+template <bool INTERIOR, bool FIRST = false>
 __device__ __forceinline__ void tile_flux(const TileView& v, const Consts<float>& k, int r, bool order2, bool visc,
                                           bool init_prims, bool last, float4* w_t, float* w_sp) {
     const Q4<float>* cq = v.cq;
@@ -294,7 +297,7 @@ __device__ __forceinline__ void tile_flux(const TileView& v, const Consts<float>
     const Q4<float>* cgy = v.cgy;
     const uint32_t sl = v.sl[r];
     const int s1 = (int)(sl & 0xFFFFu), s2 = (int)(int16_t)(sl >> 16);
-    const float4 dd = v.d[r];
+    const float4 dd = FIRST ? make_float4(0.f, 0.f, 0.f, 0.f) : v.d[r];
     const float d1x = dd.x, d1y = dd.y, d2x = dd.z, d2y = dd.w;
     const float fnx = v.nx[r], fny = v.ny[r];
     const float mxf = -fny, myf = fnx;   // unit tangent p1 -> p2
@@ -312,7 +315,7 @@ __device__ __forceinline__ void tile_flux(const TileView& v, const Consts<float>
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            L[j] = ff(g1y.p[j], d1y, ff(g1x.p[j], d1x, q1.p[j]));
+            L[j] = FIRST ? q1.p[j] : ff(g1y.p[j], d1y, ff(g1x.p[j], d1x, q1.p[j]));
             dm[j] = mm(g1y.p[j], myf, g1x.p[j], mxf);
             dq[j] = -q1.p[j];
         }
@@ -333,7 +336,7 @@ __device__ __forceinline__ void tile_flux(const TileView& v, const Consts<float>
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            Rq[j] = ff(g2y.p[j], d2y, ff(g2x.p[j], d2x, q2.p[j]));
+            Rq[j] = FIRST ? q2.p[j] : ff(g2y.p[j], d2y, ff(g2x.p[j], d2x, q2.p[j]));
             dm[j] = fm(0.5f, ff(g2y.p[j], myf, ff(g2x.p[j], mxf, dm[j])));
             dq[j] = fa(dq[j], q2.p[j]);
         }
@@ -791,6 +794,178 @@ __global__ void __launch_bounds__(kTileCore, 3) k_tstage(TArgs a) {
             red_sid = td.sid;
         }
         __syncthreads();
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// A stage of first-order solves (when every solve of the launch is one): the fluxes and the update,
+// without what only gradients need.  Such a stage is bound by latency (the descriptor, the blocks' copies,
+// the ring gather, each a round trip to L2) and has little arithmetic to hide it behind, so it takes
+// more, smaller CTAs: a tile's slots, normals, areas and the core cells' csr rows are 40 KB where the
+// general kernel's blocks and gradient rows are 73 KB, and with four CTAs of 64 registers on an SM instead
+// of three one's copies run under another's fluxes (three: 37.3 us per iteration of 300k Euler
+// polygons, four 31.7, five with spills 35.7).  One CTA per tile, no counter; each stage is launched while
+// the one before it runs (programmatic launch, triggered when every CTA of that one has started) and has
+// copied what no kernel writes when that ends (31.7 against 34.8 without the early trigger, 35.9 without
+// programmatic launches).  A tile's RK data is requested with its states, before the fluxes.
+// Against the general kernel: 300k Euler polygons 61.8 -> 31.7 us per iteration, 1M quads 136 -> 102
+// (3.3 TB/s of 110 B per cell and stage), 130k NS cylinder 44.9 -> 20.7; the same bits.
+struct TFirst {
+    int flux;                  // records with fluxes of the largest tile, rounded up to 4
+    int grad;                  // core and ring-1 cells of the largest tile
+};
+// Shared memory (bytes) of that plan: slots, normals and areas, contributions, csr, states.
+__host__ __device__ constexpr int first_smem(int flux, int grad) {
+    return 16 * flux + 16 * flux + 2 * (kTileCore + 8) + 8 * flux + 16 * grad;
+}
+static_assert(first_smem(kTileGeo, kTileGrad) <= 47 * 1024, "within the limit of a plain launch");
+
+template <int STAGE>
+__global__ void __launch_bounds__(kTileCore, 4) k_tfirst(TArgs a, TFirst f) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    float4* w_t = reinterpret_cast<float4*>(sm);
+    Q4<float>* cq = reinterpret_cast<Q4<float>*>(sm + 16 * f.flux);
+    uint32_t* ssl = reinterpret_cast<uint32_t*>(sm + 16 * f.flux + 16 * f.grad);
+    float* snx = reinterpret_cast<float*>(ssl + f.flux);
+    float* sny = snx + f.flux;
+    float* sA = sny + f.flux;
+    uint32_t* sent = reinterpret_cast<uint32_t*>(sA + f.flux);
+    uint16_t* soff = reinterpret_cast<uint16_t*>(sent + 2 * f.flux);
+    __shared__ __align__(16) TileDesc td;
+    __shared__ __align__(16) TParams tp;
+    __shared__ __align__(8) unsigned long long mbar;
+    __shared__ float redf[kTileCore / 32];
+    __shared__ float redw[4][kTileCore / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = blockIdx.x;
+    const uint32_t mb = smem_u32(&mbar);
+    if (t >= *a.ntiles) { pdl_wait(); return; }
+    if (tid < (int)(sizeof(TileDesc) / 16))
+        reinterpret_cast<int4*>(&td)[tid] = reinterpret_cast<const int4*>(a.tiles + t)[tid];
+    if (tid == 0) mbar_init(mb, 1);
+    __syncthreads();
+    const TileDesc& d = td;
+    const int nrc = d.nrc, nrc4 = (nrc + 3) & ~3, ncore = d.ncore, n1 = d.n1, ne4 = (nrc + d.ncc + 3) & ~3;
+    const int nof = (ncore + 1 + 7) & ~7;
+    if (ncore == 0) { pdl_wait(); return; }   // an empty slot of a removed solve
+    const bool ok = ncore > 0 && ncore <= kTileCore && n1 >= 0 && ncore + n1 <= f.grad && nrc >= 0 && nrc4 <= f.flux &&
+                    d.ncc >= 0 && d.ncc <= d.nint && d.nint <= nrc && nrc <= d.ngeo && d.ngeo <= d.nr && d.nrp >= nrc4 &&
+                    d.ngp >= nrc4 && nof <= d.noff && d.noff + 2 * ne4 <= d.ncsr && n1 <= d.nhalo && (d.nrp & 3) == 0 &&
+                    (d.ngp & 3) == 0 && (d.noff & 7) == 0 && (d.rec & 3) == 0 && (d.csr & 7) == 0;
+    if (!ok) {
+        if (tid == 0) atomicOr(a.err, 4);
+        pdl_wait();
+        return;
+    }
+    // what no kernel writes: the records, the csr rows and the halo ids
+    if (tid == 0) {
+        const uint32_t br = 4u * (uint32_t)nrc4, be = 4u * (uint32_t)ne4, bo = 2u * (uint32_t)nof;
+        mbar_expect_tx(mb, 4 * br + be + bo);
+        const uint32_t* rec = a.rec + d.rec;
+        const uint16_t* csr = a.csr + d.csr;
+        if (br) {
+            tma_load(ssl, rec, br, mb);
+            tma_load(snx, rec + 5 * d.nrp, br, mb);
+            tma_load(sny, rec + 5 * d.nrp + d.ngp, br, mb);
+            tma_load(sA, rec + 5 * d.nrp + 2 * d.ngp, br, mb);
+            tma_load(sent, csr + d.noff, be, mb);
+        }
+        tma_load(soff, csr, bo, mb);
+    }
+    const int c0 = d.c0, cbase = d.cbase, gid = c0 + tid;
+    const int hid = tid < n1 ? a.halo[d.halo + tid] : 0;
+    float yv = 1.f, vc = 0.f;
+    if (tid < ncore) {
+        yv = a.rvol[gid];
+        if (STAGE == 0) vc = a.vol[gid];
+    }
+    pdl_wait();   // from here on, what the stages before this one wrote
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const Q4<float>* __restrict__ Qin = a.Q[STAGE];
+    if (tid >= kTileCore - (int)(sizeof(TParams) / 16))
+        reinterpret_cast<int4*>(&tp)[tid - (kTileCore - (int)(sizeof(TParams) / 16))] =
+            reinterpret_cast<const int4*>(a.P + d.sid)[tid - (kTileCore - (int)(sizeof(TParams) / 16))];
+    Q4<float> qn, dprev, lo;
+    float dtc = 0.f, sc = 0.f;
+    if (tid < ncore) {
+        const Q4<float> q = Qin[gid];
+        cq[tid] = q;
+        if (STAGE == 0) { qn = q; sc = a.S[gid]; }
+        else { qn = a.Q[0][gid]; dprev = a.D[gid]; dtc = a.dt[gid]; }
+        if (STAGE == 2) lo = a.Qlo[gid];
+    }
+    if (tid < n1) cq[ncore + tid] = Qin[cbase + hid];
+    for (int i = tid + kTileCore; i < n1; i += kTileCore) cq[ncore + i] = Qin[cbase + a.halo[d.halo + i]];
+    const bool arrived = mbar_wait(mb, 0);
+    if (__syncthreads_or(!arrived)) {
+        if (tid == 0) atomicOr(a.err, 2);
+        return;
+    }
+    const Consts<float>& k = tp.k;
+    const bool init_prims = STAGE == 0 && tp.init_prims != 0;
+    float* w_sp = snx;   // the spectral term replaces the normal's x
+    const TileView tv{ssl, nullptr, snx, sny, sA, soff, sent, cq, nullptr, nullptr};
+    for (int r = tid; r < nrc; r += kTileCore) {
+        if (r < d.nint) tile_flux<true, true>(tv, k, r, false, false, init_prims, STAGE == 2, w_t, w_sp);
+        else tile_flux<false, true>(tv, k, r, false, false, init_prims, STAGE == 2, w_t, w_sp);
+    }
+    if (STAGE == 1 && tid == 0 && c0 == cbase) {
+        // the solve's first tile: its GLOBAL-dt maximum (read in the first stage, accumulated in the
+        // last) starts again; its history flags (read in the first stage) end
+        a.smax[d.sid] = 0.f;
+        a.P[d.sid].fresh = 0;
+        a.P[d.sid].init_prims = 0;
+    }
+    __syncthreads();
+    float snext = 0.f;
+    float r2[4] = {0.f, 0.f, 0.f, 0.f};
+    if (tid < ncore) {
+        float r4[4];
+        tile_residual(tv, tid, w_t, w_sp, STAGE == 2, yv, r4, snext);
+        if (a.R && (a.store_r || STAGE == 2)) { Q4<float> rr; for (int j = 0; j < 4; j++) rr.p[j] = r4[j]; a.R[gid] = rr; }
+        if (STAGE == 0) {
+            dtc = fm(k.two_cfl, vc) / (tp.global_dt ? a.smax[d.sid] : sc);
+            a.dt[gid] = dtc;
+        }
+        Q4<float> out, dn;
+        stage_combine(STAGE, dtc, r4, qn, dprev, lo, dn, out);
+        if (STAGE != 2) {
+            a.D[gid] = dn;
+            a.Q[STAGE + 1][gid] = out;
+        } else {
+            a.Q[0][gid] = out;
+            a.Qlo[gid] = lo;
+            a.S[gid] = snext;
+#pragma unroll
+            for (int j = 0; j < 4; j++) r2[j] = r4[j] * r4[j];
+        }
+        if (!positive(out.p[0]) || !positive(out.p[3])) atomicOr(a.flags + d.sid, 1);
+    }
+    if (STAGE == 2) {   // maxima and sums as the general kernel's: per warp, then over the warps in order
+        float m = snext;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = max2(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (a.tpart) {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) r2[j] += __shfl_xor_sync(0xffffffffu, r2[j], o);
+        }
+        if (lane == 0) {
+            redf[warp] = m;
+#pragma unroll
+            for (int j = 0; j < 4; j++) redw[j][warp] = r2[j];
+        }
+        __syncthreads();
+        if (a.tpart && tid < 4) {
+            double sum = 0.0;
+            for (int w = 0; w < kTileCore / 32; w++) sum += (double)redw[tid][w];
+            a.tpart[4 * (size_t)t + tid] = sum;
+        }
+        if (tid == 32) {
+            float bm = 0.f;
+            for (int w = 0; w < kTileCore / 32; w++) bm = max2(bm, redf[w]);
+            atomic_max_pos(a.smax + d.sid, bm);
+        }
     }
 }
 
