@@ -38,7 +38,7 @@ struct TiledImage {
     double rec_per_face = 0, ring1 = 0, ring2 = 0;
     int max_rec = 0, max_csr = 0, max_halo = 0, max_cells = 0, max_grad = 0, max_flux = 0;   // largest tile
     char* pin = nullptr;
-    size_t o_rec = 0, o_qc = 0, o_csr = 0, o_halo = 0, o_vol = 0, o_rvol = 0, o_lsq = 0;
+    size_t o_rec = 0, o_qc = 0, o_csr = 0, o_halo = 0, o_vol = 0, o_rvol = 0, o_lsq = 0, o_n2o = 0;
     ~TiledImage() { if (pin) cudaFreeHost(pin); }
 };
 
@@ -59,13 +59,13 @@ int tiled_image(const HostMesh& hm, std::shared_ptr<TiledImage>& out, std::strin
     auto take = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
     im->o_rec = take(4 * L.rec.size()); im->o_qc = take(4 * L.qcell.size()); im->o_csr = take(2 * L.csr.size());
     im->o_halo = take(4 * L.halo.size()); im->o_vol = take(4 * (size_t)L.nc4); im->o_rvol = take(4 * (size_t)L.nc4);
-    im->o_lsq = take(16 * (size_t)L.nc4);
+    im->o_lsq = take(16 * (size_t)L.nc4); im->o_n2o = take(4 * (size_t)L.nc);
     FV2D_T(cudaMallocHost(&im->pin, off));
     auto cp = [&](size_t o, const void* src, size_t bytes) { if (bytes) std::memcpy(im->pin + o, src, bytes); };
     cp(im->o_rec, L.rec.data(), 4 * L.rec.size()); cp(im->o_qc, L.qcell.data(), 4 * L.qcell.size());
     cp(im->o_csr, L.csr.data(), 2 * L.csr.size()); cp(im->o_halo, L.halo.data(), 4 * L.halo.size());
     cp(im->o_vol, L.vol.data(), 4 * (size_t)L.nc4); cp(im->o_rvol, L.rvol.data(), 4 * (size_t)L.nc4);
-    cp(im->o_lsq, L.lsq.data(), 16 * (size_t)L.nc4);
+    cp(im->o_lsq, L.lsq.data(), 16 * (size_t)L.nc4); cp(im->o_n2o, hm.cell_new2old.data(), 4 * (size_t)L.nc);
     im->tiles = std::move(L.tiles);
     im->n2o = hm.cell_new2old;
     slot = im;
@@ -866,14 +866,24 @@ private:
 // Many solves (the Batch interface).
 class TiledBatch : public Batch {
 public:
+    ~TiledBatch() override {
+        if (core_.stream_) cudaStreamSynchronize(core_.stream_);
+        for (auto e : arrived_) if (e) cudaEventDestroy(e);
+        if (stage_) cudaFreeHost(stage_);
+    }
+
     int init(long long max_cells, long long max_faces, int max_solves) override {
         if (max_cells <= 0 || max_faces <= 0 || max_solves <= 0 || max_cells > (1LL << 30) || max_faces > (1LL << 31)) {
             err_ = "batch capacity out of range (cells <= 2^30, faces <= 2^31)";
             return FV2D_ERR_ARG;
         }
         int rc = core_.init(tiled_caps(max_cells, max_faces, max_solves), false, true);
-        if (rc) err_ = core_.err;
-        return rc;
+        if (rc) { err_ = core_.err; return rc; }
+        half_ = std::min(kCopyChunk, (size_t)round_up(16 * max_cells, 256));
+        FV2D_T(cudaMallocHost(&stage_, 2 * half_ + 64));
+        flag_pin_ = (int*)(stage_ + 2 * half_);
+        for (auto& e : arrived_) FV2D_T(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        return FV2D_OK;
     }
 
     int add(const fv2d_mesh_desc* d, const fv2d_case* cs, int* sid) override {
@@ -924,15 +934,39 @@ public:
     int get_state(int sid, double* q) override {
         if (sid < 0 || sid >= core_.caps_.solves || !core_.solves_[sid].active) { err_ = "no such solve"; return FV2D_ERR_ARG; }
         const TiledCore::Solve& s = core_.solves_[sid];
-        std::vector<Q4<float>> h(s.n), lo(s.n);
-        FV2D_T(cudaStreamSynchronize(core_.stream_));
-        FV2D_T(cudaMemcpy(h.data(), core_.A_.Q[0] + s.c0, sizeof(Q4<float>) * s.n, cudaMemcpyDeviceToHost));
-        FV2D_T(cudaMemcpy(lo.data(), core_.A_.Qlo + s.c0, sizeof(Q4<float>) * s.n, cudaMemcpyDeviceToHost));
-        const std::vector<int>& n2o = s.image->n2o;
-        for (long long c = 0; c < s.n; c++)
-            for (int j = 0; j < 4; j++) q[(size_t)j * s.n + n2o[c]] = (double)h[c].p[j] + (double)lo[c].p[j];
-        int f = 0;
-        FV2D_T(cudaMemcpy(&f, core_.A_.flags + sid, 4, cudaMemcpyDeviceToHost));
+        const TArgs& A = core_.A_;
+        cudaStream_t st = core_.stream_;
+        // The device sums the state with its compensation, in the reference's numbering, into the solve's
+        // rows of the first stage's gradients, and reads the numbering from its rows of the increment: an
+        // iteration writes both before it reads them, and a batch is between iterations here.  (On the host,
+        // from two copies in device order, 96 solves of 25k cells took 15.4 ms, this way 10.6.)
+        double* out = reinterpret_cast<double*>(A.G[0] + 2 * s.c0);
+        int* n2o = reinterpret_cast<int*>(A.D + s.c0);
+        FV2D_T(cudaMemcpyAsync(n2o, s.image->pin + s.image->o_n2o, 4 * (size_t)s.n, cudaMemcpyHostToDevice, st));
+        k_state_out<float><<<(unsigned)((s.n + 255) / 256), 256, 0, st>>>((int)s.n, 4, n2o, A.Q[0] + s.c0, out, A.Qlo + s.c0);
+        FV2D_T(cudaGetLastError());
+        FV2D_T(cudaMemcpyAsync(flag_pin_, A.flags + sid, 4, cudaMemcpyDeviceToHost, st));
+        const size_t bytes = 32 * (size_t)s.n;
+        if (host_pinned(q)) {
+            FV2D_T(cudaMemcpyAsync(q, out, bytes, cudaMemcpyDeviceToHost, st));
+            FV2D_T(cudaStreamSynchronize(st));
+        } else {
+            // through two page-locked halves: the host copies one piece while the next arrives
+            auto fetch = [&](size_t off) {
+                const size_t n = std::min(half_, bytes - off), h = (off / half_) & 1;
+                cudaError_t e = cudaMemcpyAsync(stage_ + h * half_, (const char*)out + off, n, cudaMemcpyDeviceToHost, st);
+                return e == cudaSuccess ? cudaEventRecord(arrived_[h], st) : e;
+            };
+            if (bytes) FV2D_T(fetch(0));
+            for (size_t off = 0; off < bytes; off += half_) {
+                const size_t n = std::min(half_, bytes - off), h = (off / half_) & 1;
+                if (off + half_ < bytes) FV2D_T(fetch(off + half_));
+                FV2D_T(cudaEventSynchronize(arrived_[h]));
+                CopyPool::get().copy((char*)q + off, stage_ + h * half_, n);
+            }
+            FV2D_T(cudaStreamSynchronize(st));
+        }
+        const int f = *flag_pin_;
         if (f) { err_ = "non-physical state (rho <= 0, E <= 0 or NaN) in this solve"; return FV2D_ERR_STATE; }
         return FV2D_OK;
     }
@@ -983,6 +1017,10 @@ public:
 private:
     TiledCore core_;
     BatchTuning tune_;
+    char* stage_ = nullptr;   // page-locked: two halves for state transfers, a solve's flag
+    size_t half_ = 0;
+    int* flag_pin_ = nullptr;
+    cudaEvent_t arrived_[2] = {nullptr, nullptr};
 };
 
 #undef FV2D_T

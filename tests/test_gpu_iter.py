@@ -119,3 +119,24 @@ def test_handles_of_different_plans_in_turn(pkg):
         assert bits_equal(s.get_state(), t.get_state())
         t.close()
         s.close()
+
+
+@pytest.mark.parametrize("timing", [False, True])   # whole-iteration kernel, stage kernels
+def test_batch_states_between_iterations(pkg, timing):
+    """get_state() between iterations (it works in rows that the next iteration writes first) leaves the
+    run as it is, for first- and second-order solves, and returns the freestream of a solve not yet stepped."""
+    cases = [(pkg.meshgen.channel_bump_quads(31, 12), case_of(pkg, eqn="EULER")),
+             (pkg.meshgen.voronoi_bump_channel(5000, seed=2), case_of(pkg, eqn="NS", mu=0.02, BC1="NO_SLIP_WALL")),
+             (pkg.meshgen.channel_bump_quads(9, 30), case_of(pkg, eqn="EULER", solution_poly_order=0, limiter="NONE"))]
+    b = pkg.Batch(20000, 60000, 4, precision=pkg.FP32)
+    b.set_kernel_timing(timing)
+    ids = [b.add(g, c) for g, c in cases]
+    solvers = [pkg.Solver(g, c, precision=pkg.FP32) for g, c in cases]
+    for n in (0, 1, 3, 2):
+        b.step(n)
+        for i, s in zip(ids, solvers):
+            s.step(n)
+            assert bits_equal(b.get_state(i), s.get_state())
+    for s in solvers:
+        s.close()
+    b.close()
