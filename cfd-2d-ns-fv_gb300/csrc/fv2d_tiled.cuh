@@ -174,8 +174,12 @@ struct TileView {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // The limited LSQ gradient of one core or ring-1 cell (local slot gI).  ghost(r): the state of the
-// cell that a no-slip face's gradient ghost reads; prev(): the cell's previous-stage state.
-template <class Ghost, class Prev>
+// cell that a no-slip face's gradient ghost reads; prev(): the cell's previous-stage state.  PAIRS: warps
+// without boundary faces take two faces at a time, whose extremes cost one three-operand minimum or
+// maximum each instead of two (the stage kernels, bound by issue: 1M-cell NS cylinder 304.0 ->
+// 298.4 us per iteration, 600k quads 157.0 -> 155.9; the whole-iteration kernel, bound by latency, is faster without:
+// 50k Euler polygons 19.46 against 19.69).
+template <bool PAIRS, class Ghost, class Prev>
 __device__ __forceinline__ void tile_gradient(const TileView& v, const Consts<float>& k, int gI, bool squeeze, bool lim_prev,
                                               bool init_prims, bool stage0, const float4& mom, const Q4<float>& gpx,
                                               const Q4<float>& gpy, Ghost ghost, Prev prev, Q4<float>& gx, Q4<float>& gy) {
@@ -196,9 +200,9 @@ __device__ __forceinline__ void tile_gradient(const TileView& v, const Consts<fl
     // branches
     const uint32_t o1 = v.off[gI + 1];
     const int e0 = v.off[gI] & 0x7FFF, e1 = (int)(o1 & 0x7FFFu);
-    auto face_loop = [&](auto interior) {
+    auto face_loop = [&](auto interior, int first) {
         constexpr bool INTERIOR = decltype(interior)::value;
-        for (int e = e0; e < e1; e++) {
+        for (int e = first; e < e1; e++) {
             const uint32_t ent = v.ent[e];
             const int r = (int)((ent & 0xFFFFu) >> 1), side = (int)(ent & 1u);
             const int so = (int)(int16_t)(ent >> 16);   // the face's other cell (or BC code)
@@ -255,8 +259,34 @@ __device__ __forceinline__ void tile_gradient(const TileView& v, const Consts<fl
     };
     // one loop per warp: the general one if any of its cells has a boundary face (a warp running
     // both would take the sum of the two)
-    if (__any_sync(__activemask(), (o1 & 0x8000u) != 0)) face_loop(std::false_type{});
-    else face_loop(std::true_type{});
+    if (__any_sync(__activemask(), (o1 & 0x8000u) != 0)) face_loop(std::false_type{}, e0);
+    else if (!PAIRS) face_loop(std::true_type{}, e0);
+    else {
+        int e = e0;
+        for (; e + 1 < e1; e += 2) {
+            const uint32_t ea = v.ent[e], eb = v.ent[e + 1];
+            const float4 da = v.d[(ea & 0xFFFFu) >> 1], db = v.d[(eb & 0xFFFFu) >> 1];
+            const Q4<float> qa = v.cq[(int)(int16_t)(ea >> 16)], qb = v.cq[(int)(int16_t)(eb >> 16)];
+            const bool sa = ea & 1u, sb = eb & 1u;
+            // as above: the face centre from this cell (o) and the displacement to the other's (f)
+            const float oxa = sa ? da.z : da.x, oya = sa ? da.w : da.y, oxb = sb ? db.z : db.x, oyb = sb ? db.w : db.y;
+            const float fxa = fs(oxa, sa ? da.x : da.z), fya = fs(oya, sa ? da.y : da.w);
+            const float fxb = fs(oxb, sb ? db.x : db.z), fyb = fs(oyb, sb ? db.y : db.w);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float a = fs(qa.p[j], qc.p[j]), b = fs(qb.p[j], qc.p[j]);
+                sx[j] = ff(b, fxb, ff(a, fxa, sx[j]));
+                sy[j] = ff(b, fyb, ff(a, fya, sy[j]));
+                if (squeeze) { dmin[j] = fminf(fminf(a, b), dmin[j]); dmax[j] = fmaxf(fmaxf(a, b), dmax[j]); }
+                if (lim_prev) {
+                    const float x = mm(gpx.p[j], oxa, gpy.p[j], oya), y = mm(gpx.p[j], oxb, gpy.p[j], oyb);
+                    tmin[j] = fminf(fminf(x, y), tmin[j]);
+                    tmax[j] = fmaxf(fmaxf(x, y), tmax[j]);
+                }
+            }
+        }
+        face_loop(std::true_type{}, e);
+    }
     const float ixx = mom.x, iyy = mom.y, ixy = mom.z;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -663,7 +693,7 @@ __global__ void __launch_bounds__(kTileCore, 3) k_tstage(TArgs a) {
             Q4<float> gpx, gpy;
             if (lim_prev) { gpx = Gprev[2 * (size_t)gid]; gpy = Gprev[2 * (size_t)gid + 1]; }
             Q4<float> gx, gy;
-            tile_gradient(tv, k, gI, squeeze, lim_prev, init_prims, STAGE == 0, mom, gpx, gpy,
+            tile_gradient<true>(tv, k, gI, squeeze, lim_prev, init_prims, STAGE == 0, mom, gpx, gpy,
                           [&](int r) { return Qin[cbase + a.qcell[td.rbase + r]]; }, [&] { return Qprev[gid]; }, gx, gy);
             cg[gI] = gx;
             cgy[gI] = gy;
@@ -1119,7 +1149,7 @@ __global__ void __launch_bounds__(kTileCore, MINB) k_titer(TArgs a, TIter it) {
                 for (int gI = tid; gI < ncore + n1; gI += blockDim.x) {
                     Q4<float> gpx, gpy, gx, gy;
                     if (lim_prev) { gpx = cg[gI]; gpy = cgy[gI]; }
-                    tile_gradient(tv, k, gI, squeeze, lim_prev, init_prims, s == 0, slsq[gI], gpx, gpy,
+                    tile_gradient<false>(tv, k, gI, squeeze, lim_prev, init_prims, s == 0, slsq[gI], gpx, gpy,
                                   [&](int r) { return ldcg_q(Qin + cbase + a.qcell[td.rbase + r]); }, [&] { return sqp[gI]; }, gx, gy);
                     cg[gI] = gx;
                     cgy[gI] = gy;
