@@ -11,7 +11,8 @@
 //           [ncore, ncore+n1) ring 1, [ncore+n1, ncore+n1+n2) ring 2; halo[] lists ring 1 then ring 2
 //   records one per face the tile needs: [0, nrc) every face of a core cell (fluxes are computed for
 //           these; the first ncc join two core cells, the first nint join two cells, the rest are
-//           boundary faces), [nrc, ngeo) boundary faces of ring-1 cells,
+//           boundary faces; within the first two groups in an order that spares shared-memory bank
+//           conflicts), [nrc, ngeo) boundary faces of ring-1 cells,
 //           [ngeo, nr) the other faces of ring-1 cells (gradient only).  Record block, 4-byte words:
 //             sl[nrp]   (s1 & 0xFFFF) | (s2 << 16): local slots of the face's c1 and c2 (s2 < 0: BC code)
 //             d[nrp][4] (d1x, d1y, d2x, d2y): face centre minus c1 / c2 centre (c2: ghost centre for
