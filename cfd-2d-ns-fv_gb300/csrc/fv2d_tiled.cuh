@@ -463,7 +463,9 @@ __device__ __forceinline__ void tile_flux(const TileView& v, const Consts<float>
 }
 
 // Residual of core cell c (res.cpp:74-109): its faces' contributions in ascending original face id,
-// over its volume (yv = 1/vol); on the last stage its spectral terms' sum too.
+// over its volume (yv = 1/vol); on the last stage its spectral terms' sum too.  The side's sign enters
+// as an exact factor of a multiply-add, which costs no operation of its own (300k first-order
+// polygons 30.13 -> 29.63 us per iteration).
 __device__ __forceinline__ void tile_residual(const TileView& v, int c, const float4* w_t, const float* w_sp, bool last,
                                               float yv, float r4[4], float& snext) {
 #pragma unroll
@@ -471,12 +473,13 @@ __device__ __forceinline__ void tile_residual(const TileView& v, int c, const fl
     const int e0 = v.off[c] & 0x7FFF, e1 = v.off[c + 1] & 0x7FFF;
     for (int e = e0; e < e1; e++) {
         const uint32_t ent = v.ent[e];
-        const int r = (int)((ent & 0xFFFFu) >> 1), side = (int)(ent & 1u);
+        const int r = (int)((ent & 0xFFFFu) >> 1);
         const float4 tv = w_t[r];
-        r4[0] = fa(r4[0], neg_if(tv.x, side));
-        r4[1] = fa(r4[1], neg_if(tv.y, side));
-        r4[2] = fa(r4[2], neg_if(tv.z, side));
-        r4[3] = fa(r4[3], neg_if(tv.w, side));
+        const float sg = __uint_as_float((ent << 31) | 0x3F800000u);   // +1 or, on the face's second side, -1
+        r4[0] = ff(tv.x, sg, r4[0]);
+        r4[1] = ff(tv.y, sg, r4[1]);
+        r4[2] = ff(tv.z, sg, r4[2]);
+        r4[3] = ff(tv.w, sg, r4[3]);
         if (last) snext = fa(snext, w_sp[r]);
     }
 #pragma unroll
