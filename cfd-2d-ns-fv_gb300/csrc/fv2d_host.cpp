@@ -429,7 +429,7 @@ int build_mesh(const fv2d_mesh_desc* d, const fv2d_case* cs, HostMesh& m, std::s
     return FV2D_OK;
 }
 
-void build_layout(const HostMesh& m, DeviceLayout& L) {
+void build_layout(const HostMesh& m, DeviceLayout& L, bool tiles) {
     const int nc = m.nc, nf = m.nf;
     L.nc = nc; L.nf = nf;
     L.inc_off.assign(nc + 1, 0);
@@ -438,7 +438,8 @@ void build_layout(const HostMesh& m, DeviceLayout& L) {
         L.inc_off[i + 1] = L.inc_off[i] + (m.cf_off[o + 1] - m.cf_off[o]);
     }
     L.ninc = L.inc_off[nc];
-    L.inc.resize(L.ninc); L.nbr.resize(L.ninc); L.igeo.resize(4 * (size_t)L.ninc);
+    L.inc.resize(L.ninc);
+    if (!tiles) { L.nbr.resize(L.ninc); L.igeo.resize(4 * (size_t)L.ninc); }
     for (int i = 0; i < nc; i++) {
         const int o = m.cell_new2old[i];
         int w = L.inc_off[i];
@@ -446,6 +447,7 @@ void build_layout(const HostMesh& m, DeviceLayout& L) {
             const int f = m.cf[k];
             const int side = (m.fc1[f] == o) ? 0 : 1;
             L.inc[w] = (m.face_old2new[f] << 1) | side;
+            if (tiles) continue;
             L.igeo[4 * (size_t)w + 0] = m.dxj[f];
             L.igeo[4 * (size_t)w + 1] = m.dyj[f];
             L.igeo[4 * (size_t)w + 2] = side == 0 ? m.c1dx[f] : m.c2dx[f];
@@ -455,7 +457,8 @@ void build_layout(const HostMesh& m, DeviceLayout& L) {
         }
     }
     L.fc1.resize(nf); L.fc2.resize(nf); L.qcell.resize(nf);
-    for (int g = 0; g < 14; g++) L.fgeo[g].resize(nf);
+    const int ngeo = tiles ? 7 : 14;
+    for (int g = 0; g < ngeo; g++) L.fgeo[g].resize(nf);
     const std::vector<double>* src[14] = {&m.nx, &m.ny, &m.area, &m.c1dx, &m.c1dy, &m.c2dx, &m.c2dy,
                                           &m.dxj, &m.dyj, &m.mx, &m.my, &m.lx, &m.ly, &m.dist};
     for (int i = 0; i < nf; i++) {
@@ -463,7 +466,7 @@ void build_layout(const HostMesh& m, DeviceLayout& L) {
         L.fc1[i] = m.cell_old2new[m.fc1[f]];
         L.fc2[i] = m.fc2[f] >= 0 ? m.cell_old2new[m.fc2[f]] : m.fc2[f];
         L.qcell[i] = (m.fc2[f] == FV2D_BC_NO_SLIP_WALL) ? m.cell_old2new[f] : -1;
-        for (int g = 0; g < 14; g++) L.fgeo[g][i] = (*src[g])[f];
+        for (int g = 0; g < ngeo; g++) L.fgeo[g][i] = (*src[g])[f];
     }
     L.vol.resize(nc); L.Ixx.resize(nc); L.Iyy.resize(nc); L.Ixy.resize(nc);
     for (int i = 0; i < nc; i++) {

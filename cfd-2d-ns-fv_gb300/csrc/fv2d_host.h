@@ -58,7 +58,8 @@ int write_grid(const char* path, const fv2d_mesh_desc* d, std::string& err);
 // Device order of cells and faces: Hilbert order, cells by face count within runs of `block` cells.
 constexpr int kSideBlock = 256;
 int build_mesh(const fv2d_mesh_desc* d, const fv2d_case* cs, HostMesh& m, std::string& err, int block = kSideBlock);
-void build_layout(const HostMesh& m, DeviceLayout& L);
+// tiles: only what the tile layout of the FP32 engine takes (no nbr, igeo, fgeo[7..13])
+void build_layout(const HostMesh& m, DeviceLayout& L, bool tiles = false);
 int mesh_field(const HostMesh& m, int field, double* out);
 
 }  // namespace fv2d

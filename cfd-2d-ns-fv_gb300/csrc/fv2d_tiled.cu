@@ -46,7 +46,7 @@ int tiled_image(const HostMesh& hm, std::shared_ptr<TiledImage>& out, std::strin
     auto& slot = hm.batch_image[1];
     if (slot) { out = std::static_pointer_cast<TiledImage>(slot); return FV2D_OK; }
     DeviceLayout D;
-    build_layout(hm, D);
+    build_layout(hm, D, true);
     TileLayout L;
     if (!build_tile_layout(hm, D, L, err, core)) return FV2D_ERR_MESH;
     auto im = std::make_shared<TiledImage>();

@@ -53,7 +53,7 @@ constexpr int kRecRun = 128;
 // memory wavefronts drop from 1.87 to 1.54 of the least possible on Voronoi meshes (runs of 64: 1.58; whole
 // groups: 1.47 and 0.4% less time a stage, but the search for a row's record grows with the run) and from 1.96 to 1.66 on quads:
 // 1M-cell NS cylinder 298.4 -> 290.0 us per iteration, 600k quads 155.9 -> 152.9, 300k first-order
-// polygons 31.7 -> 30.2.  Results do not depend on the order; building a mesh's tiles takes 6% longer.
+// polygons 31.7 -> 30.2.  Results do not depend on the order; the order takes 2% of a solver's creation on the host.
 void order_records(Tile& t, Marks& mk) {
     const int nr = (int)t.faces.size(), ncore = t.ncore, ngrad = ncore + (int)t.ring1.size();
     auto& rec = mk.rec;
@@ -89,15 +89,20 @@ void order_records(Tile& t, Marks& mk) {
             const int r1 = std::min(r0 + kRecRun, lim[part + 1]);
             int cap[8] = {0, 0, 0, 0, 0, 0, 0, 0}, cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             for (int r = r0; r < r1; r++) cap[r & 7]++;
+            uint16_t taken[8];   // past every cost when full
+            for (int c = 0; c < 8; c++) taken[c] = cap[c] ? 0 : 4096;
             for (int r = r0; r < r1; r++) {
                 const Marks::Rec& x = rec[r];
                 const uint64_t cost = (met[x.at[0]] << x.w[0]) + (met[x.at[1]] << x.w[1]);
-                int best = 0, bc = 1 << 30;
-                for (int c = 0; c < 8; c++) {
-                    const int k = (int)((cost >> (8 * c)) & 255u) * 64 + cnt[c] + (cnt[c] == cap[c] ? 1 << 20 : 0);
-                    if (k < bc) { best = c; bc = k; }
-                }
+                // (least cost, then fewest taken, then the residue) as one word per residue
+                uint16_t word[8];
+                for (int c = 0; c < 8; c++)
+                    word[c] = (uint16_t)(((((cost >> (8 * c)) & 255u) * 32 + taken[c]) << 3) | (unsigned)c);
+                uint16_t least = word[0];
+                for (int c = 1; c < 8; c++) least = std::min(least, word[c]);
+                const int best = least & 7;
                 cls[best][cnt[best]++] = r;
+                taken[best] = cnt[best] == cap[best] ? 4096 : (uint16_t)cnt[best];
                 met[x.at[0]] += (uint64_t)1 << (8 * best);
                 met[x.at[1]] += (uint64_t)1 << (8 * best);
             }
