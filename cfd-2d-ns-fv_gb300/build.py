@@ -50,7 +50,7 @@ def _units():
         # FP32 values are far above FP32's normal range; norms are summed in FP64)
         ("fv2d_tiled.cu", [nvcc] + common + ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]),
         # (on the host too: Arm compilers contract by default, and this freestream state is the oracle's only
-        # uncontracted.  The engine above keeps its compiler's default: with the SQUEEZE limiter a batch's run from
+        # uncontracted.  fv2d_fp64.cu keeps the compiler's default: with the SQUEEZE limiter a batch's run from
         # the uniform freestream magnifies an ulp of it to 1e-5, so its bits are kept from version to version)
         ("fv2d_noalloc.cu", [nvcc] + common + ["-fmad=false", "-Xcompiler", "-ffp-contract=off"]),
     ]

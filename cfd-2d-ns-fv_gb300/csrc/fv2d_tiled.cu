@@ -238,7 +238,10 @@ public:
         iter_smem_ = off;
         iter_planned_ = true;
         iter_fn_ = nullptr;
-        if (hi_tiles_ <= 0) return FV2D_OK;
+        // First-order solves run faster by stage kernels at every size: a stage of theirs launched as a programmatic
+        // dependent costs 2.5 us, the grid barrier and ring gather here alone about as much (2k Euler polygons
+        // 7.4 us per iteration against 8.8, 50k 10.0 against 13.0, 85k 13.1 against 18.5)
+        if (hi_tiles_ <= 0 || first_) return FV2D_OK;
         // two CTAs per SM (no spills) where that holds every tile, else three
         for (const void* f : {(const void*)k_titer<2>, (const void*)k_titer<3>}) {
             int per = 0;
