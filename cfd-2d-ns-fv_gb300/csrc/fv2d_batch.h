@@ -1,6 +1,6 @@
 // Precision-agnostic interface of the batched engine: many independent solves resident in one
-// device arena, advanced together by persistent tile kernels (one launch per kernel per RK stage,
-// one CUDA graph per iteration).  Solves can join and leave between iterations.
+// device arena, advanced together by tile kernels (one launch per kernel per RK stage replayed as CUDA
+// graphs, or whole iterations in one launch).  Solves can join and leave between iterations.
 #pragma once
 
 #include <string>

@@ -982,7 +982,8 @@ public:
 
     // The FP32 engine's tiles are fixed by its layout (up to 256 cells, one CTA of 256 threads per
     // tile); its tuning is, per solve-size bucket, the faces per warp of the flux pass (flux records a
-    // warp takes per grab: 32 x tile_mult) and the grid mode (persistent CTAs, or one CTA per tile).
+    // warp takes per grab: 32 x tile_mult) and the grid mode (persistent CTAs, or one CTA per tile); both act
+    // on the general stage kernel only.
     // `block` is validated and kept but does not change the launch.
     int set_tuning(const BatchTuning& t) override {
         if (t.block < 64 || t.block > 256 || (t.block & 31)) { err_ = "block must be a multiple of 32 in [64, 256]"; return FV2D_ERR_ARG; }

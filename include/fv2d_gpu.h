@@ -187,8 +187,8 @@ const char* fv2d_last_error(fv2d_handle* h);   /* h may be NULL: last creation e
  * advances exactly as ssp_rk3() (src/solver/ssp_rk3.cpp:18) would advance it alone.  A batch owns
  * one device arena sized at creation (cells, faces, solves); solves are added (mesh + case, the
  * same inputs as fv2d_create) and removed between iterations; fv2d_batch_step advances every
- * active solve together with one persistent launch per kernel per RK stage, replayed as one CUDA
- * graph per iteration.  Per-solve residual L2 norms of the last iteration support retirement.
+ * active solve together with one launch per kernel per RK stage, replayed as CUDA graphs (FP32
+ * batches whose tiles all fit on the GPU: whole iterations in one launch).  Per-solve residual L2 norms of the last iteration support retirement.
  * Errors: fv2d_last_error(NULL).                                                                 */
 typedef struct fv2d_batch fv2d_batch;
 int fv2d_batch_create(long long max_cells, long long max_faces, int max_solves, int precision, fv2d_batch** out);
@@ -211,7 +211,9 @@ int fv2d_batch_synchronize(fv2d_batch* b);
  * results never depend on it.  FP64: threads per block (a multiple of 32 in [64, 256]) and tiles
  * of block * tile_mult[bucket] elements.  FP32 (fused stage kernel over the mesh's 256-cell tiles,
  * 256 threads per tile): block is not used; tile_mult[bucket] in [1, 32] sets the faces per warp of
- * the flux pass (32 * tile_mult flux records per grab).                                          */
+ * the flux pass (32 * tile_mult flux records per grab), where the batch runs the general stage kernel:
+ * batches whose tiles all fit on the GPU at once run whole iterations in one launch, and batches of
+ * first-order solves their own stage kernel, neither of which takes the tuning.                   */
 int fv2d_batch_set_tuning(fv2d_batch* b, int block, const int* tile_mult3, const int* bucket_edges2);
 int fv2d_batch_get_tuning(fv2d_batch* b, int* block, int* tile_mult3, int* bucket_edges2);
 /* grid of the stage kernels: 0 = persistent (SMs x resident blocks loop over the tiles),
