@@ -93,6 +93,13 @@ private:
 
 constexpr size_t kCopyChunk = size_t(8) << 20;
 
+// Bytes of the staging buffer of a solver that uploads its mesh arrays and moves its fields through
+// it: the largest single transfer.  A field is up to 8 doubles per cell; the norm partials, 4 doubles
+// per block of the reduction, are more than that on meshes of less than half as many cells as blocks.
+inline size_t solver_staging_bytes(size_t cells, size_t faces, size_t incidences, size_t norm_blocks, size_t real) {
+    return std::max<size_t>({8 * 8 * cells, 4 * (cells + 1), real * faces, 4 * faces, 4 * incidences, 8 * 4 * norm_blocks});
+}
+
 // Page-locked (cudaMallocHost / cudaHostRegister) host memory can be the DMA endpoint itself.
 inline bool host_pinned(const void* p) {
     cudaPointerAttributes a;

@@ -116,9 +116,8 @@ public:
         D_ = comp ? (Q4<T>*)(a + o_D) : nullptr;
         Qlo_ = comp ? (Q4<T>*)(a + o_lo) : nullptr;
         FV2D_CUDA(cudaMemsetAsync(arena_, 0, arena_bytes_, stream_));
-        // ---- upload (one pinned staging buffer reused for every array)
-        staging_bytes_ = std::max<size_t>({sizeof(T) * (size_t)nf_, 8 * (size_t)nc_ * 8, 4 * (size_t)ninc_,
-                                           4 * (size_t)(nc_ + 1), 4 * (size_t)nf_});
+        // ---- upload (one pinned staging buffer reused for every array, the fields and the norm partials)
+        staging_bytes_ = solver_staging_bytes(nc_, nf_, ninc_, nred_, sizeof(T));
         FV2D_CUDA(cudaMallocHost(&host_stage_, staging_bytes_));
         FV2D_CUDA(cudaEventCreateWithFlags(&stage_free_, cudaEventDisableTiming));
         auto put = [&](void* dst, const void* src, size_t bytes) -> int {
