@@ -914,7 +914,7 @@ __global__ void __launch_bounds__(kTileCore, 4) k_tfirst(TArgs a, TFirst f) {
     }
     pdl_wait();   // from here on, what the stages before this one wrote
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const Q4<float>* __restrict__ Qin = a.Q[STAGE];
+    const Q4<float>* Qin = a.Q[STAGE];   // not __restrict__: it changes while this kernel is resident
     if (tid >= kTileCore - (int)(sizeof(TParams) / 16))
         reinterpret_cast<int4*>(&tp)[tid - (kTileCore - (int)(sizeof(TParams) / 16))] =
             reinterpret_cast<const int4*>(a.P + d.sid)[tid - (kTileCore - (int)(sizeof(TParams) / 16))];
