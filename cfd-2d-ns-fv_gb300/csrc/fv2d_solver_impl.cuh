@@ -192,9 +192,12 @@ public:
     // Qbar only; face histories and the stage counter are kept (the run continues).
     int load_state(const double* q) override {
         if (stage_ != 0) { err_ = "load_state between iterations only (stage counter is not 0)"; return FV2D_ERR_ARG; }
-        FV2D_CUDA(staged_h2d(dstage_, q, 8 * 4 * (size_t)nc_, host_stage_, stream_, stage_free_));
+        bool reading = false;
+        FV2D_CUDA(staged_h2d(dstage_, q, 8 * 4 * (size_t)nc_, host_stage_, stream_, stage_free_, &reading));
         launch(K_STATE_IN, nc_, [&](int gr) { k_state_in<T><<<gr, 256, 0, stream_>>>(nc_, n2o_, dstage_, Q_[0], Qlo_); });
         FV2D_CUDA(cudaGetLastError());
+        // the caller may write its buffer as soon as this returns
+        if (reading) FV2D_CUDA(cudaEventSynchronize(stage_free_));
         init_prims_ = false;
         return FV2D_OK;
     }

@@ -137,7 +137,8 @@ int fv2d_set_state(fv2d_handle* h, const double* q);
 /* Replace Qbar by q (4N, SoA, file numbering) WITHOUT resetting the face histories the next
  * stage reads (previous-stage face values, Vn_avg/c_avg).  For a host loop that hands back the
  * state it read with fv2d_get_state, as the reference's main() hands Qbar to ssp_rk3() every
- * iteration (src/base/main.cpp:126): upload, step, download continues the run exactly.        */
+ * iteration (src/base/main.cpp:126): upload, step, download continues the run exactly.
+ * Both calls have taken q, page-locked or not, when they return: the caller may write it again. */
 int fv2d_load_state(fv2d_handle* h, const double* q);
 /* Copy Qbar back (4N, SoA, file numbering).                                                    */
 int fv2d_get_state(fv2d_handle* h, double* q);
