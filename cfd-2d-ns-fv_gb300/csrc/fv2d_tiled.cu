@@ -485,14 +485,20 @@ public:
         return FV2D_OK;
     }
 
+    // The kernels' error word (TArgs::err) as a status: such a kernel left its tiles unfinished.
+    static int kernel_status(int e, std::string& err) {
+        if (e & 2) { err = "a stage kernel's wait for its tile copies timed out"; return FV2D_ERR_CUDA; }
+        if (e & 4) { err = "a tile descriptor is out of range"; return FV2D_ERR_CUDA; }
+        if (e & 8) { err = "a barrier between the tiles timed out"; return FV2D_ERR_CUDA; }
+        return FV2D_OK;
+    }
+
     // Device status: CUDA errors, a kernel's timeout / descriptor error, non-physical states.
     int check(int* flags_out, int nflags) {
         FV2D_T(cudaStreamSynchronize(stream_));
         int e = 0;
         FV2D_T(cudaMemcpy(&e, A_.err, 4, cudaMemcpyDeviceToHost));
-        if (e & 2) { err = "a stage kernel's wait for its tile copies timed out"; return FV2D_ERR_CUDA; }
-        if (e & 4) { err = "a tile descriptor is out of range"; return FV2D_ERR_CUDA; }
-        if (e & 8) { err = "a barrier between the tiles timed out"; return FV2D_ERR_CUDA; }
+        if (int rc = kernel_status(e, err)) return rc;
         if (flags_out && nflags > 0) FV2D_T(cudaMemcpy(flags_out, A_.flags, 4 * (size_t)nflags, cudaMemcpyDeviceToHost));
         return FV2D_OK;
     }
@@ -949,6 +955,7 @@ public:
         k_state_out<float><<<(unsigned)((s.n + 255) / 256), 256, 0, st>>>((int)s.n, 4, n2o, A.Q[0] + s.c0, out, A.Qlo + s.c0);
         FV2D_T(cudaGetLastError());
         FV2D_T(cudaMemcpyAsync(flag_pin_, A.flags + sid, 4, cudaMemcpyDeviceToHost, st));
+        FV2D_T(cudaMemcpyAsync(flag_pin_ + 1, A.err, 4, cudaMemcpyDeviceToHost, st));
         const size_t bytes = 32 * (size_t)s.n;
         if (host_pinned(q)) {
             FV2D_T(cudaMemcpyAsync(q, out, bytes, cudaMemcpyDeviceToHost, st));
@@ -969,7 +976,8 @@ public:
             }
             FV2D_T(cudaStreamSynchronize(st));
         }
-        const int f = *flag_pin_;
+        const int f = flag_pin_[0];
+        if (int rc = TiledCore::kernel_status(flag_pin_[1], err_)) return rc;
         if (f) { err_ = "non-physical state (rho <= 0, E <= 0 or NaN) in this solve"; return FV2D_ERR_STATE; }
         return FV2D_OK;
     }
@@ -1021,7 +1029,7 @@ public:
 private:
     TiledCore core_;
     BatchTuning tune_;
-    char* stage_ = nullptr;   // page-locked: two halves for state transfers, a solve's flag
+    char* stage_ = nullptr;   // page-locked: two halves for state transfers, a solve's flag and the kernels' error word
     size_t half_ = 0;
     int* flag_pin_ = nullptr;
     cudaEvent_t arrived_[2] = {nullptr, nullptr};

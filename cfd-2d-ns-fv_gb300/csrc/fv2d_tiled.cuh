@@ -59,7 +59,7 @@ struct TArgs {
     int nsmax;                 // entries of smax
     int* flags;                // [solves] non-physical state seen
     double* tpart;             // [tiles][4] residual sums of squares of the last stage (null: none)
-    int* err;                  // bit 1: an mbarrier wait timed out; bit 2: a tile descriptor out of range
+    int* err;                  // 2: an mbarrier wait timed out; 4: a tile descriptor out of range; 8: a grid barrier timed out
     int store_r;               // keep R on stages 0 and 1 too
 };
 
