@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "fv2d_batch.h"
@@ -942,6 +943,8 @@ public:
 
     int get_state(int sid, double* q) override {
         if (sid < 0 || sid >= core_.caps_.solves || !core_.solves_[sid].active) { err_ = "no such solve"; return FV2D_ERR_ARG; }
+        // one read-back at a time: threads that fetch different solves share the staging halves and the flag
+        std::lock_guard<std::mutex> lock(transfer_);
         const TiledCore::Solve& s = core_.solves_[sid];
         const TArgs& A = core_.A_;
         cudaStream_t st = core_.stream_;
@@ -1032,6 +1035,7 @@ private:
     char* stage_ = nullptr;   // page-locked: two halves for state transfers, a solve's flag and the kernels' error word
     size_t half_ = 0;
     int* flag_pin_ = nullptr;
+    std::mutex transfer_;
     cudaEvent_t arrived_[2] = {nullptr, nullptr};
 };
 
