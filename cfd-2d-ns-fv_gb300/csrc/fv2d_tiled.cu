@@ -384,15 +384,16 @@ public:
         return FV2D_OK;
     }
 
-    // One stage kernel over every tile.
-    int launch_stage(int st) {
+    // One stage kernel over every tile (general: also where the active solves are all first order).
+    int launch_stage(int st, bool general = false) {
+        const bool first = first_ && !general;
         // (the stage's tile counter was zeroed by the previous stage's kernel; the GLOBAL-dt maxima
         // by the second stage's)
         timed(st, [&] {
             // persistent grid (CTAs that take tiles until none is left) or one CTA per tile slot (always
             // of the first-order kernel)
-            const int gr = full_grid_ || first_ ? (int)std::max<long long>(1, hi_tiles_) : grid_;
-            if (first_) {
+            const int gr = full_grid_ || first ? (int)std::max<long long>(1, hi_tiles_) : grid_;
+            if (first) {
                 TFirst f = first_plan_;
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3((unsigned)gr);
@@ -446,7 +447,14 @@ public:
     // CUDA-graph replays (captured once; the graphs read the tile list from
     // device memory, so solves join and leave without re-capture): runs of kGraphIters iterations
     // as one replay (fewer gaps between replays), the rest one iteration per replay.
+    // A caller's capture of the handle's stream takes the general stage kernels: k_titer's barrier word
+    // counts the launches that ran, which a graph replayed any number of times does not follow, and
+    // the others' grids and plans are those of the solves active now.
     int iterations(int n, bool graphs) {
+        cudaStreamCaptureStatus capture_status;
+        FV2D_T(cudaStreamIsCapturing(stream_, &capture_status));
+        const bool captured = capture_status != cudaStreamCaptureStatusNone;
+        if (captured) graphs = false;
         int it = 0;
         if (n > 0 && graphs && !timing_) {
             int rc = iter_planned_ ? FV2D_OK : plan_iter();
@@ -457,7 +465,7 @@ public:
         while (it < n) {
             int k = 1;
             if (!graphs || timing_) {
-                for (int st = 0; st < 3; st++) { int rc = launch_stage(st); if (rc) return rc; }
+                for (int st = 0; st < 3; st++) { int rc = launch_stage(st, captured); if (rc) return rc; }
             } else {
                 const int w = n - it >= kGraphIters ? 1 : 0;
                 k = w ? kGraphIters : 1;
