@@ -183,25 +183,24 @@ struct Fp {
 // a - b*q0 is exact and q0 + (a - b*q0)*y rounds to the correctly rounded a/b (Markstein, as above:
 // y correctly rounded, q0 faithful).  Four operations a quotient and two per denominator, against
 // five for the two residual corrections of Recip.  Same operand range; a zero numerator gives the exact
-// signed zero.  Tested bit for bit against IEEE division.
+// signed zero, or NaN over a zero.  Tested bit for bit against IEEE division.
 struct Divisor {
     double b, y, yl;
+    int z;   // high word of +0 / b: b's sign, over NaN's bits where b is a zero (a state of no density is then flagged)
     __device__ __forceinline__ Divisor(double b_, double y_, const Fp& f) {
         b = b_;
         y = y_;
         yl = f.mul(__fma_rn(-b_, y_, f.one), y_);
+        const int hb = __double2hiint(b_);
+        z = (hb & (int)0x80000000) | (((hb << 1) | __double2loint(b_)) == 0 ? 0x7FF80000 : 0);
     }
-    __device__ __forceinline__ Divisor(double b_, const Fp& f) {
-        b = b_;
-        y = __drcp_rn(b_);
-        yl = f.mul(__fma_rn(-b_, y, f.one), y);
-    }
+    __device__ __forceinline__ Divisor(double b_, const Fp& f) : Divisor(b_, Recip<double>::of(b_), f) {}
     __device__ __forceinline__ double div(double a, const Fp& f) const {
         const double q0 = __fma_rn(a, y, f.mul(a, yl));
         const double q = __fma_rn(__fma_rn(-b, q0, a), y, q0);
         const int ha = __double2hiint(a);
         const bool zero = ((ha << 1) | __double2loint(a)) == 0;
-        return zero ? __hiloint2double((ha ^ __double2hiint(b)) & (int)0x80000000, 0) : q;
+        return zero ? __hiloint2double((ha & (int)0x80000000) ^ z, 0) : q;
     }
 };
 
