@@ -259,7 +259,10 @@ void* fv2d_batch_stream(fv2d_batch* b);
  * -4 (NO_SLIP_WALL); cell_face_offsets non-decreasing from 0; cell_faces holds
  * (face id << 1) | side (side 1 when the cell is face_cell2) with face ids in [0, num_faces), in
  * ascending face id per cell, which reproduces the reference's summation order; q and r are SoA
- * p1..p4 blocks of num_cells doubles.  From the case only gamma, the [init] state and
+ * p1..p4 blocks of num_cells doubles.  States are not checked: zero or infinite components and NaN
+ * give the infinities and NaN of IEEE arithmetic.  Results are those of the plain expressions bit for bit
+ * while density and quotients are normal doubles and nothing comes within a factor of 4 of overflow;
+ * beyond that the last bits may differ.  From the case only gamma, the [init] state and
  * flux_solver are read (RUSANOV only: ROE is rejected with FV2D_ERR_CASE). */
 #define FV2D_NOALLOC_MAX_FACES 262144
 typedef struct fv2d_noalloc_mesh {
