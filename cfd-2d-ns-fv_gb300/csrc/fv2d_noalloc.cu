@@ -172,8 +172,10 @@ k_noalloc_face(int nf, const int* __restrict__ fc1, const int* __restrict__ fc2,
 __global__ void __launch_bounds__(128)
 k_noalloc_gather(int nc, const int* __restrict__ off, const int* __restrict__ inc, const double* __restrict__ vol,
                  const double* __restrict__ scratch, double* __restrict__ r) {
-    const int c = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 2), j = threadIdx.x & 3;
-    if (c >= nc) return;
+    // (not the thread's index over 4, which wraps from 2^30 cells on; cells without faces count too)
+    const unsigned cell = blockIdx.x * (blockDim.x >> 2) + (threadIdx.x >> 2);
+    if (cell >= (unsigned)nc) return;
+    const int c = (int)cell, j = threadIdx.x & 3;
     const Fp fp;
     const int b = off[c], e = off[c + 1];
     const double v = vol[c];
