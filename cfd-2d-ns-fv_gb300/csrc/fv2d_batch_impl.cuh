@@ -6,7 +6,7 @@
 // Work is described by tile lists in device memory (tile = up to `block * mult` cells or faces of
 // one solve); each stage kernel is a persistent grid looping over its tiles, loads the solve's
 // parameters into shared memory once per tile and applies the same per-element code.  One
-// iteration (3 stages x 3 kernels + 2 memsets) is captured in a CUDA graph; since the graph reads
+// iteration (3 stages x 3 kernels, a memset and the norms) is captured in a CUDA graph; since the graph reads
 // the tile lists and parameter table from device memory, solves can join and leave between
 // iterations without re-capturing.  Per-solve reductions: the GLOBAL dt maximum uses one atomic
 // max per tile (a maximum does not depend on the order); the residual L2 sums are written per tile
@@ -52,14 +52,9 @@ __device__ __forceinline__ T block_max_t(T v, T* red) {
     return s;   // valid in thread 0
 }
 
-// Largest block the batch kernels accept (the autotuner's largest) and the FP32 kernels' minimum
-// resident blocks at that size (their register caps: gradient 64, face 48 - measured fastest);
-// FP64 keeps a 128-register cap.
+// Largest block the batch kernels accept (the autotuner's largest), at a 128-register cap.
 #ifndef FV2D_KB_MAXT
 #define FV2D_KB_MAXT 256
-#endif
-#ifndef FV2D_KBG_MINB32
-#define FV2D_KBG_MINB32 4
 #endif
 constexpr int kBatchMaxBlock = FV2D_KB_MAXT;
 constexpr int kBatchMinB64 = 512 / FV2D_KB_MAXT;
@@ -67,7 +62,7 @@ constexpr int kBatchMinB64 = 512 / FV2D_KB_MAXT;
 #define FV2D_KBG_MINB64 kBatchMinB64
 #endif
 template <class T>
-__global__ void __launch_bounds__(FV2D_KB_MAXT, sizeof(T) == 4 ? FV2D_KBG_MINB32 : FV2D_KBG_MINB64)
+__global__ void __launch_bounds__(FV2D_KB_MAXT, FV2D_KBG_MINB64)
 kb_gradient(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevMesh<T> m,
             const SolveParams<T>* __restrict__ P, const Q4<T>* __restrict__ Qin, Q4<T>* __restrict__ Gout) {
     __shared__ SolveParams<T> sp;
@@ -88,11 +83,8 @@ kb_gradient(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevM
     }
 }
 
-#ifndef FV2D_KBF_MINB32
-#define FV2D_KBF_MINB32 5
-#endif
 template <class T, bool LAST>
-__global__ void __launch_bounds__(FV2D_KB_MAXT, sizeof(T) == 4 ? FV2D_KBF_MINB32 : kBatchMinB64)
+__global__ void __launch_bounds__(FV2D_KB_MAXT, kBatchMinB64)
 kb_face(const Tile* __restrict__ tiles, const int* __restrict__ ntiles, DevMesh<T> m,
         const SolveParams<T>* __restrict__ P, const Q4<T>* __restrict__ Qin, const Q4<T>* __restrict__ G,
         Q4<T>* __restrict__ tout, T* __restrict__ sout) {
@@ -224,13 +216,10 @@ __global__ void k_shift_ids(I* __restrict__ inc_off, int n1, I i0, I* __restrict
     }
 }
 
-// A newly admitted solve's uniform initial state (and its FP32 compensation term).
+// A newly admitted solve's uniform initial state.
 template <class T>
-__global__ void k_fill_q(Q4<T>* __restrict__ Q, Q4<T>* __restrict__ Qlo, int n, Q4<T> hi, Q4<T> lo) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        Q[i] = hi;
-        if (Qlo) Qlo[i] = lo;
-    }
+__global__ void k_fill_q(Q4<T>* __restrict__ Q, int n, Q4<T> q) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) Q[i] = q;
 }
 
 #define FV2D_B(call)                                                                              \
@@ -293,12 +282,9 @@ public:
         size_t ot = take(q4 * Fc_), os = take(sizeof(T) * Fc_);
         size_t oP = take(sizeof(SolveParams<T>) * S_), osmax = take(sizeof(T) * S_), ores = take(32 * (size_t)S_);
         size_t oflag = take(4 * (size_t)S_);
-        const bool comp = sizeof(T) == 4;   // FP32: delta-form increments + compensated base state
-        size_t oD = comp ? take(q4 * Nc_) : 0, olo = comp ? take(q4 * Nc_) : 0;
-        // FP64: the face pass stores its reconstructed face states for the next squeeze (as the
-        // single-solve FP64 engine does); a solve's first stage after admission uses the sentinel
-        const bool fv = !comp;
-        size_t ofval = fv ? take(2 * q4 * Fc_) : 0;
+        // the face pass stores its reconstructed face states for the next squeeze (as the single-solve
+        // engine does); a solve's first stage after admission uses the sentinel
+        size_t ofval = take(2 * q4 * Fc_);
         tile_cap_ = (int)std::min<long long>((Nc_ + Fc_) / 64 + 4 * (long long)S_ + 16, 1LL << 28);
         size_t otc = take(sizeof(Tile) * tile_cap_), otf = take(sizeof(Tile) * tile_cap_), ocnt = take(64);
         size_t otp = take(32 * (size_t)tile_cap_), osr = take(8 * (size_t)S_);
@@ -316,8 +302,6 @@ public:
         P_ = (SolveParams<T>*)(a + oP); smax_ = (T*)(a + osmax); res2_ = (double*)(a + ores); flags_ = (int*)(a + oflag);
         tc_ = (Tile*)(a + otc); tf_ = (Tile*)(a + otf); cnt_ = (int*)(a + ocnt);
         tpart_ = (double*)(a + otp); srange_ = (int*)(a + osr);
-        D_ = comp ? (Q4<T>*)(a + oD) : nullptr;
-        Qlo_ = comp ? (Q4<T>*)(a + olo) : nullptr;
         m_.inc_off = incoff; m_.inc = inc; m_.nbr = nbr; m_.fc1 = fc1; m_.fc2 = fc2; m_.qcell = qc;
         m_.igeo = (const Q4<T>*)(a + oigeo);
         m_.g.nx = geo_[0]; m_.g.ny = geo_[1]; m_.g.area = geo_[2]; m_.g.c1dx = geo_[3]; m_.g.c1dy = geo_[4];
@@ -325,7 +309,7 @@ public:
         m_.g.my = geo_[10]; m_.g.lx = geo_[11]; m_.g.ly = geo_[12]; m_.g.dist = geo_[13];
         m_.Ixx = ixx; m_.Iyy = iyy; m_.Ixy = ixy; m_.vol = vol;
         m_.rvol = (T*)(a + orvol); m_.rdist = (T*)(a + ordist);
-        m_.fval = fv ? (Q4<T>*)(a + ofval) : nullptr;
+        m_.fval = (Q4<T>*)(a + ofval);
         FV2D_B(cudaMemsetAsync(arena_, 0, bytes_, stream_));
         FV2D_B(cudaStreamSynchronize(stream_));
         cells_.reset(Nc_);
@@ -460,13 +444,12 @@ public:
         p.global_dt = cs->time_type == FV2D_DT_GLOBAL; p.fresh = 1; p.init_prims = 1;
         pin_params_[sid] = p;   // a slot is rewritten only after its solve was removed (synchronised)
         FV2D_B(cudaMemcpyAsync(P_ + sid, pin_params_ + sid, sizeof(p), cudaMemcpyHostToDevice, stream_));
-        // as the single-solve upload: hi = the state rounded to T, lo = the rounded remainder
         const double qd[4] = {cs->rho, cs->rho * cs->u, cs->rho * cs->v, E};
-        Q4<T> hi1, lo1;
-        for (int j = 0; j < 4; j++) { hi1.p[j] = (T)qd[j]; lo1.p[j] = (T)(qd[j] - (double)hi1.p[j]); }
+        Q4<T> q0;
+        for (int j = 0; j < 4; j++) q0.p[j] = (T)qd[j];
         {
             const int gr = (int)std::min<long long>((r.n + 255) / 256, 4LL * sms_);
-            k_fill_q<T><<<gr, 256, 0, stream_>>>(Q_[0] + r.c0, Qlo_ ? Qlo_ + r.c0 : nullptr, (int)r.n, hi1, lo1);
+            k_fill_q<T><<<gr, 256, 0, stream_>>>(Q_[0] + r.c0, (int)r.n, q0);
             FV2D_B(cudaGetLastError());
         }
         FV2D_B(cudaMemsetAsync(flags_ + sid, 0, 4, stream_));
@@ -544,14 +527,12 @@ public:
     int get_state(int sid, double* q) override {
         if (sid < 0 || sid >= S_ || !recs_[sid].active) { err_ = "no such solve"; return FV2D_ERR_ARG; }
         const Rec& r = recs_[sid];
-        std::vector<Q4<T>> h(r.n), lo(Qlo_ ? r.n : 0);
+        std::vector<Q4<T>> h(r.n);
         FV2D_B(cudaStreamSynchronize(stream_));
         FV2D_B(cudaMemcpy(h.data(), Q_[0] + r.c0, sizeof(Q4<T>) * r.n, cudaMemcpyDeviceToHost));
-        if (Qlo_) FV2D_B(cudaMemcpy(lo.data(), Qlo_ + r.c0, sizeof(Q4<T>) * r.n, cudaMemcpyDeviceToHost));
         for (long long c = 0; c < r.n; c++) {
             const int o = r.n2o[c];
-            for (int j = 0; j < 4; j++)   // FP64: the value itself (adding 0.0 would turn -0 into +0)
-                q[(size_t)j * r.n + o] = Qlo_ ? (double)h[c].p[j] + (double)lo[c].p[j] : (double)h[c].p[j];
+            for (int j = 0; j < 4; j++) q[(size_t)j * r.n + o] = (double)h[c].p[j];
         }
         int f = 0;
         FV2D_B(cudaMemcpy(&f, flags_ + sid, 4, cudaMemcpyDeviceToHost));
@@ -740,8 +721,6 @@ private:
     T *dt_ = nullptr, *S_arr_ = nullptr, *s_ = nullptr, *smax_ = nullptr;
     T* geo_[14] = {nullptr};
     Q4<T>* t_ = nullptr;
-    Q4<T>* D_ = nullptr;     // FP32 only: RK increment in delta form
-    Q4<T>* Qlo_ = nullptr;   // FP32 only: compensation term of Qn
     SolveParams<T>* P_ = nullptr;
     double* res2_ = nullptr;
     double* tpart_ = nullptr;   // per cell tile: residual sums of squares of the last stage

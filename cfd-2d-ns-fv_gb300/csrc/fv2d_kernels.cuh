@@ -2,10 +2,11 @@
 // helpers both precisions share, templated on the state type T).
 //
 // One RK stage = three launches:
-//   k_gradient  (one thread per cell)  LSQ gradient over the cell's faces + squeeze limiter
-//   k_face      (one thread per face)  reconstruction, boundary ghosts, NS face terms, Rusanov
-//                                      flux; writes the face's residual contribution
-//   k_update    (one thread per cell)  gathers the face contributions in ascending original face
+//   k_gradient  (four lanes per cell)  LSQ gradient over the cell's faces + squeeze limiter, one
+//                                      component per lane
+//   k_face      (one thread per face;  reconstruction, boundary ghosts, NS face terms, Rusanov
+//    k_face_pair: two lanes)           flux; writes the face's residual contribution
+//   k_update    (four lanes per cell)  gathers the face contributions in ascending original face
 //                                      id, divides by the volume, applies the SSP-RK3 stage, and
 //                                      (last stage) the spectral sums for the next time step
 // Every per-cell sum visits the cell's faces in ascending ORIGINAL face id, the order in which
@@ -55,8 +56,7 @@ struct DevMesh {
     const T *rdist, *rvol;
     // reconstructed face states of the last face pass, [2 nf]: 2f + side (the incidence code) holds
     // the state on cell c1's (side 0) or c2's (side 1) side of face f - exactly the stale face
-    // values the next squeeze reads.  Null: the squeeze recomputes them from the previous stage's
-    // state and limited gradient with the same expression.
+    // values the next squeeze reads.  Null where no squeeze follows.
     Q4<T>* fval;
 };
 
@@ -101,17 +101,6 @@ __device__ __forceinline__ T min2(T a, T b) { return less(b, a) ? b : a; }
 template <class T>
 __device__ __forceinline__ T max2(T a, T b) { return less(a, b) ? b : a; }
 
-// class_Q::updateflow for one state (class_q.hpp:131-141); T (temperature) is never read by the
-// step and is not formed.
-template <class T>
-__device__ __forceinline__ void prims(const T p[4], const Consts<T>& k, T& rho, T& u, T& v, T& P) {
-    rho = p[0];
-    const T E = p[3];
-    u = p[1] / rho;
-    v = p[2] / rho;
-    P = (E - (T(0.5) * rho * (u * u + v * v))) * k.gm1;
-}
-
 // Division sharing one reciprocal between several quotients with the same denominator.
 // FP64: y = RN(1/b) (__drcp_rn), then two of Markstein's residual corrections
 // (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
@@ -121,12 +110,8 @@ __device__ __forceinline__ void prims(const T p[4], const Consts<T>& k, T& rho, 
 // normal operands whose quotient neither overflows nor underflows (all solver quantities); a zero
 // numerator (checked on its bits, not with an FP64 compare) returns the exact signed zero a*y.
 // Tested bit for bit against IEEE division.
-// FP32 divides directly (the FP32 engine is built with approximate division).
 template <class T>
-struct Recip {
-    static __device__ __forceinline__ T of(T b) { return T(1) / b; }
-    static __device__ __forceinline__ T div(T a, T b, T) { return a / b; }
-};
+struct Recip;
 template <>
 struct Recip<double> {
     static __device__ __forceinline__ double of(double b) { return __drcp_rn(b); }
@@ -138,16 +123,13 @@ struct Recip<double> {
     }
 };
 
-// a/3.  FP64: one residual correction suffices for this divisor (two are needed in general).
+// a/3: one residual correction suffices for this divisor (two are needed in general).
 // y = RN(1/3) = 1/3 (1 - 2^-54), so a*y is within half an ulp of a/3 and q0 = RN(a*y) is faithful;
 // r = a - 3 q0 is then exact (an integer multiple of ulp(q0), below 3 ulp), and q0 + r*y is within
 // 2^-53 ulp of a/3.  a/3 lies at least ulp/6 from every rounding midpoint (a - 3m, m a midpoint,
 // is a non-zero multiple of ulp/2), so RN(q0 + r*y) is the correctly rounded a/3.  Checked against
 // IEEE division on the host (tests/cpu_helpers/div3_check.cpp).
-template <class T>
-__device__ __forceinline__ T div3(T a) { return Recip<T>::div(a, T(3), T(1.0 / 3.0)); }
-template <>
-__device__ __forceinline__ double div3<double>(double a) {
+__device__ __forceinline__ double div3(double a) {
     const double y = 1.0 / 3.0, q0 = a * y;
     if ((__double_as_longlong(a) << 1) == 0) return q0;   // a == +-0
     return __fma_rn(__fma_rn(-3.0, q0, a), y, q0);
@@ -160,9 +142,9 @@ __device__ __forceinline__ double div3<double>(double a) {
 // exactly as a + b and a*b do, signed zeros included: a*1 is exact, and adding -0 changes no value and
 // no zero's sign.  The constants have to come from memory: from literals or kernel parameters the
 // compiler rebuilds the slower forms.
-// Together with the exact scalings of face_flux, on the 1M-cell NS cylinder: face kernel 2.19 -> 1.75 ms
-// (FP64 pipe busy 94.5 % of the time), gradient 0.40 -> 0.38, update 0.135 -> 0.115; 8.37 -> 6.87 ms per
-// iteration.
+// Together with the exact scalings of face_flux, on the 1M-cell NS cylinder: face kernel 2.20 -> 1.76 ms
+// (FP64 pipe busy 95 % of the time); with the component lanes of the cell passes gradient 0.459 -> 0.431,
+// update 0.141 -> 0.146 (below), 8.37 -> 6.99 ms per iteration.
 // half: a factor of 1/2 enters through the multiply-add that uses it (x - m/2 = fma(m, -1/2, x), as
 // m/2 is exact), so it costs no operation of its own.
 __device__ double g_fp64_consts[4] = {1.0, -0.0, 0.5, 0.25};
@@ -210,12 +192,9 @@ __device__ __forceinline__ double zero_minus(double x) {
     const long long b = __double_as_longlong(x) ^ (long long)0x8000000000000000ULL;
     return (b << 1) == 0 ? 0.0 : __longlong_as_double(b);
 }
-__device__ __forceinline__ float zero_minus(float x) {
-    const int b = __float_as_int(x) ^ (int)0x80000000u;
-    return (b << 1) == 0 ? 0.0f : __int_as_float(b);
-}
 
-// prims() with rho's divisor shared by u, v (and returned for P/rho)
+// Primitives of one state (class_Q::updateflow, class_q.hpp:131-141; T, the temperature, is never read by the
+// step and is not formed): rho's divisor is shared by u and v, and returned for P/rho.
 __device__ __forceinline__ Divisor prims_r(const double p[4], const Consts<double>& k, const Fp& f, double& u, double& v,
                                            double& P) {
     const Divisor r(p[0], f);
@@ -239,9 +218,8 @@ __device__ __forceinline__ void cons(T rho, T u, T v, T P, const Consts<T>& k, T
 // Gradient + squeeze limiter.  compute_gradient (src/solver/cell_gradient.cpp:9-131) and
 // squeeze (src/solver/squeeze.cpp:9-155), restated as one gather per cell.
 // The squeeze compares against the face values of the PREVIOUS stage (res.cpp:40 runs before the
-// reconstruction at :48); they are recomputed here from the previous stage's state and limited
-// gradient with the reconstruction's own expression, or are the -101 sentinel the face states
-// start with (class_q.hpp:73-76) on the first stage after initialisation.
+// reconstruction at :48): those its face pass stored (DevMesh::fval), or the -101 sentinel the face
+// states start with (class_q.hpp:73-76) on the first stage after initialisation.
 // a[j] for a run-time j without indexing (which would put the array in local memory)
 template <class T>
 __device__ __forceinline__ T pick4(const T a[4], int j) {
@@ -407,7 +385,8 @@ __device__ __forceinline__ double first_order_state(double q, double dx, double 
 // state's sums S = L + R stand for 2 (L + R)/2, the wave speed t = |vn1 + vn2| + (c1 + c2) for 4 lambda,
 // the flux F2 for 2 F against half the area, the viscous flux V2 for 2 V (mu and k enter doubled), and
 // the remaining halves ride on multiply-adds.  Every rounded intermediate is the reference's times a
-// power of two, so the results are the same bits.  338 FP64 operations for an NS interior face.
+// power of two, so the results are the same bits.  352 FP64 pipe slots for an NS face (356 on the last stage),
+// 160 for an Euler face, those of the reciprocals and roots included.
 template <bool ORDER2, bool NS, bool LAST, class Wait>
 __device__ __forceinline__ void face_flux(int f, const Fp& fp, const DevMesh<double>& m, const Q4<double>* Q,
                                           const Q4<double>* G, Q4<double>* tout, double* sout, const Consts<double>& k,
@@ -651,7 +630,6 @@ __device__ __forceinline__ double spectral_sum(const int* __restrict__ inc, cons
 __device__ __forceinline__ double neg_if(double x, int s) {
     return __longlong_as_double(__double_as_longlong(x) ^ ((long long)s << 63));
 }
-__device__ __forceinline__ float neg_if(float x, int s) { return __int_as_float(__float_as_int(x) ^ (s << 31)); }
 
 // x > 0 (false for NaN).  FP64 on the integer pipe: 0 < bits <= bits(+inf).
 template <class T>
@@ -724,8 +702,10 @@ __device__ __forceinline__ double update_lane(int c, int j, const Fp& fp, const 
 
 // Threads per block of the update kernel: four lanes (one component each) per cell; the block's first
 // warp also holds one lane per cell for what a cell needs once: its time step in the first stage
-// (one division) and its spectral sum in the last.  The second stage, which does not read it, zeroes
-// the spectral maximum that the last accumulates.
+// (one division) and its spectral sum in the last.  Large meshes, where the pipe and not the chain is the
+// limit, pay for it: each lane repeats the incidence loop's and the division's overhead (66 -> 73 pipe
+// slots per cell; 300k cells 43.3 -> 45.3 us, 1M 141 -> 146), against 20 us less in the gradient at 300k.
+// The second stage, which does not read it, zeroes the spectral maximum that the last accumulates.
 constexpr int kUpdBlock = 128, kUpdCells = kUpdBlock / 4;
 
 template <int STAGE>
@@ -765,8 +745,8 @@ k_update(int nc, DevMesh<double> m, const Q4<double>* tface, const double* sface
 // that the length of a lane's chain of operations is the pass's time: lane h = 0 takes cell c1's side, components 0
 // and 1 of the flux and the x derivatives, lane h = 1 cell c2's side, components 2 and 3 and the y
 // derivatives.  Every value is computed by the expression face_flux uses, so the bits are the same;
-// about 205 operations a lane for an NS interior face against 352.  All 32 lanes call (act: the lane
-// pair has a face).  (With programmatic launches: 512 Euler quads 58 -> 50 us per iteration, 2k NS
+// 204 FP64 pipe slots a lane for an NS face against 352, 88 against 160 for an Euler face.  All 32 lanes
+// call (act: the lane pair has a face).  (With programmatic launches: 512 Euler quads 58 -> 50 us per iteration, 2k NS
 // polygons 80 -> 72; with two warps to a quarter the extra work loses, 8k NS polygons 118 -> 131.)
 template <bool ORDER2, bool NS>
 __device__ __forceinline__ void face_pair(int f, int h, bool act, const Fp& fp, const DevMesh<double>& m, const Q4<double>* Q,

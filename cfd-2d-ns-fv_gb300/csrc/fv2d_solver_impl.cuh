@@ -1,4 +1,4 @@
-// Solver engine for one precision: device arena, stage sequencing, CUDA-graph replay of whole
+// Solver engine, FP64 (T = double): device arena, stage sequencing, CUDA-graph replay of whole
 // iterations, per-kernel event timing and host<->device field transfers.
 #pragma once
 
@@ -83,15 +83,12 @@ public:
         size_t o_t = take(q4 * nf_), o_s = take(sizeof(T) * nf_);
         size_t o_smax = take(64), o_flag = take(64);
         size_t o_n2o = take(4 * (size_t)nc_);
-        // FP64 squeeze: the face pass stores its reconstructed states for the next limiter pass
-        // (the FP32 engine, memory-bound, recomputes them instead)
-        const bool store_fval = sizeof(T) == 8 && order2_ && squeeze_;
+        // squeeze: the face pass stores its reconstructed states for the next limiter pass
+        const bool store_fval = order2_ && squeeze_;
         size_t o_fval = store_fval ? take(2 * q4 * (size_t)nf_) : 0;
         size_t o_stage = take(8 * 8 * (size_t)nc_);
         nred_ = 304;
         size_t o_part = take(8 * 4 * (size_t)nred_);
-        const bool comp = sizeof(T) == 4;   // FP32: delta-form increments + compensated base state
-        size_t o_D = comp ? take(q4 * nc_) : 0, o_lo = comp ? take(q4 * nc_) : 0;
         arena_bytes_ = off;
         FV2D_CUDA(cudaMalloc(&arena_, arena_bytes_));
         char* a = (char*)arena_;
@@ -113,8 +110,6 @@ public:
         dm_.fval = store_fval ? (Q4<T>*)(a + o_fval) : nullptr;
         smax_ = (T*)(a + o_smax); flag_ = (int*)(a + o_flag);
         n2o_ = (int*)(a + o_n2o); dstage_ = (double*)(a + o_stage); part_ = (double*)(a + o_part);
-        D_ = comp ? (Q4<T>*)(a + o_D) : nullptr;
-        Qlo_ = comp ? (Q4<T>*)(a + o_lo) : nullptr;
         FV2D_CUDA(cudaMemsetAsync(arena_, 0, arena_bytes_, stream_));
         // ---- upload (one pinned staging buffer reused for every array, the fields and the norm partials)
         staging_bytes_ = solver_staging_bytes(nc_, nf_, ninc_, nred_, sizeof(T));
@@ -173,7 +168,7 @@ public:
 
     int upload_state(const double* q) {
         FV2D_CUDA(staged_h2d(dstage_, q, 8 * 4 * (size_t)nc_, host_stage_, stream_, stage_free_));
-        launch(K_STATE_IN, nc_, [&](int gr) { k_state_in<T><<<gr, 256, 0, stream_>>>(nc_, n2o_, dstage_, Q_[0], Qlo_); });
+        launch(K_STATE_IN, nc_, [&](int gr) { k_state_in<T><<<gr, 256, 0, stream_>>>(nc_, n2o_, dstage_, Q_[0], nullptr); });
         // fresh face histories: -101 sentinel for the limiter, initial Vn_avg/c_avg for dt
         FV2D_CUDA(cudaMemsetAsync(smax_, 0, 64, stream_));
         launch(K_SPECTRAL, nc_, [&](int gr) {
@@ -194,7 +189,7 @@ public:
         if (stage_ != 0) { err_ = "load_state between iterations only (stage counter is not 0)"; return FV2D_ERR_ARG; }
         bool reading = false;
         FV2D_CUDA(staged_h2d(dstage_, q, 8 * 4 * (size_t)nc_, host_stage_, stream_, stage_free_, &reading));
-        launch(K_STATE_IN, nc_, [&](int gr) { k_state_in<T><<<gr, 256, 0, stream_>>>(nc_, n2o_, dstage_, Q_[0], Qlo_); });
+        launch(K_STATE_IN, nc_, [&](int gr) { k_state_in<T><<<gr, 256, 0, stream_>>>(nc_, n2o_, dstage_, Q_[0], nullptr); });
         FV2D_CUDA(cudaGetLastError());
         // the caller may write its buffer as soon as this returns
         if (reading) FV2D_CUDA(cudaEventSynchronize(stage_free_));
@@ -292,8 +287,7 @@ public:
             launch(K_STATE_OUT, nc_, [&](int gr) { k_scalar_out<T><<<gr, 256, 0, stream_>>>(nc_, n2o_, (const T*)src, dstage_); });
         else
             launch(K_STATE_OUT, nc_, [&](int gr) {
-                k_state_out<T><<<gr, 256, 0, stream_>>>(nc_, ncomp, n2o_, (const Q4<T>*)src, dstage_,
-                                                         field == FV2D_F_QBAR ? Qlo_ : nullptr);
+                k_state_out<T><<<gr, 256, 0, stream_>>>(nc_, ncomp, n2o_, (const Q4<T>*)src, dstage_, nullptr);
             });
         const size_t bytes = 8 * (size_t)ncomp * nc_;
         FV2D_CUDA(staged_d2h(out, dstage_, bytes, host_stage_, stream_, copy_events_));
@@ -418,8 +412,6 @@ private:
     Q4<T>* Q_[3] = {nullptr, nullptr, nullptr};
     Q4<T>* G_[3] = {nullptr, nullptr, nullptr};
     Q4<T>* R_ = nullptr;
-    Q4<T>* D_ = nullptr;     // FP32 only: RK increment in delta form
-    Q4<T>* Qlo_ = nullptr;   // FP32 only: compensation term of Qn
     Q4<T>* t_ = nullptr;
     T *dt_ = nullptr, *S_ = nullptr, *vol_ = nullptr, *s_ = nullptr, *smax_ = nullptr;
     double *Ixx_ = nullptr, *Iyy_ = nullptr, *Ixy_ = nullptr, *dstage_ = nullptr, *part_ = nullptr;
