@@ -41,17 +41,17 @@ def _units():
         ("fv2d_tiles.cpp", host),
         ("fv2d_output.cpp", host),
         ("fv2d_api.cu", [nvcc] + common),
-        # the FP64 engine must not contract a*b+c: bit-identical with the reference
+        # the FP64 engine's device code must not contract a*b+c: bit-identical with the reference.  Its host code
+        # keeps the compiler's default, and GCC contracts on Arm: there the freestream energy P/(gamma-1) +
+        # rho(u*u+v*v)/2 is an ulp off the reference's for about 5% of inputs.  Kept so that results stay the
+        # same from version to version: from a uniform start the SQUEEZE limiter magnifies that ulp to 1e-5
         ("fv2d_fp64.cu", [nvcc] + common + ["-fmad=false"]),
-        # the FP32 engine: a single solve and a batch run the same fused stage kernels, so FMA
-        # contraction is allowed (both round alike); divisions and square roots use the
-        # approximate (few-ulp) forms
-        # FP32 engine: approximate division and square root, denormals flushed to zero (the flow's
-        # FP32 values are far above FP32's normal range; norms are summed in FP64)
+        # the FP32 engine: its shared passes round as written (explicit products and multiply-adds), so every
+        # kernel gives the same bits; elsewhere contraction is allowed.  Approximate division and square root,
+        # denormals flushed to zero (the flow's FP32 values are far above FP32's normal range; norms are
+        # summed in FP64)
         ("fv2d_tiled.cu", [nvcc] + common + ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]),
-        # (on the host too: Arm compilers contract by default, and this freestream state is the oracle's only
-        # uncontracted.  fv2d_fp64.cu keeps the compiler's default: with the SQUEEZE limiter a batch's run from
-        # the uniform freestream magnifies an ulp of it to 1e-5, so its bits are kept from version to version)
+        # (no contraction on the host either: this entry's freestream state is the reference's on Arm too)
         ("fv2d_noalloc.cu", [nvcc] + common + ["-fmad=false", "-Xcompiler", "-ffp-contract=off"]),
     ]
 

@@ -1,8 +1,8 @@
 // FP32 engine: state, gradients and fluxes in FP32 (the LSQ moments stay FP64, the residual norms
 // are accumulated in FP64), one fused kernel per SSP-RK3 stage over the tile layout
 // (fv2d_tiles.h, fv2d_tiled.cuh).  A single solve (TiledSolver, the Solver interface) and a batch of
-// independent solves (TiledBatch, the Batch interface) run on the same core and the same kernels,
-// so a solve gives the same bits alone and in a batch; FMA contraction is therefore allowed here.
+// independent solves (TiledBatch, the Batch interface) run on the same core and the same passes, whose
+// operations round as written, so a solve gives the same bits alone and in a batch.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -86,7 +86,10 @@ int tiled_image(const HostMesh& hm, std::shared_ptr<TiledImage>& out, std::strin
 // / 256: 22.1 / 23.9 / 25.8 (43.5); 88k, 196 (three per SM): 31.7 (44.8).
 // Beyond that the stage kernels take the tiles in waves of three per SM; with only two waves the
 // second is filled by cutting the tiles evenly (120k polygons: 256 -> 136 cells 75.7 -> 66.7 us;
-// 180k: 256 -> 200 76.4 -> 71.6).  From three waves on smaller tiles cost as much in ring cells as the
+// 180k: 256 -> 200 76.4 -> 71.6).  One wave that three CTAs per SM hold with larger tiles (91,201 to 116,736
+// cells) keeps 256 cells; cut evenly 95k polygons take 40.1 -> 39.5, 105k 41.6 -> 40.4, 115k 41.6 -> 42.0.
+// (The line of 200 cells is that of polygons; quads need less shared memory and could go further.)
+// From three waves on smaller tiles cost as much in ring cells as the
 // fuller last wave gains (300k: 116.4 -> 116.2; 1M quads 252 -> 258 at 248 cells).
 int solve_tile_cells(long long n, int sms) {
     auto even = [&](long long tiles) { return (int)round_up((n + tiles - 1) / tiles, 4); };

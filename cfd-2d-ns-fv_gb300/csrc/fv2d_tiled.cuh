@@ -836,14 +836,14 @@ __global__ void __launch_bounds__(kTileCore, 3) k_tstage(TArgs a) {
 // the ring gather, each a round trip to L2) and has little arithmetic to hide it behind, so it takes
 // more, smaller CTAs: a tile's slots, normals, areas and the core cells' csr rows are 40 KB where the
 // general kernel's blocks and gradient rows are 73 KB, and with four CTAs of 64 registers on an SM instead
-// of three one's copies run under another's fluxes (three: 37.3 us per iteration of 300k Euler
-// polygons, four 31.7, five with spills 35.7).  One CTA per tile, no counter; each stage is launched while
+// of three one's copies run under another's fluxes.  One CTA per tile, no counter; each stage is launched while
 // the one before it runs (programmatic launch, triggered when every CTA of that one has started) and has
-// copied what no kernel writes when that ends (31.7 against 34.8 without the early trigger; with five CTAs
-// 35.7, 37.8 and, without programmatic launches, 39.0).  A tile's RK data is requested with its states, before the fluxes.
-// Against the general kernel: 300k Euler polygons 62.9 -> 29.8 us per iteration, 1M quads 137 -> 98
-// (about 145 B per cell and stage: 4.4 TB/s), 130k NS cylinder 45.2 -> 19.7; the same bits.  (The
-// variants' figures above are from before the records were ordered for the banks.)
+// copied what no kernel writes when that ends.  A tile's RK data is requested with its states, before the fluxes.
+// Against the general kernel: 300k Euler polygons 62.9 -> 29.4 us per iteration, 1M quads 137 -> 99
+// (about 145 B per cell and stage: 4.4 TB/s), 130k NS cylinder 45.2 -> 19.5; the same bits.
+// The choices, measured on 300k Euler polygons when the kernel took 31.7 (its records not yet ordered for the
+// banks): three CTAs per SM 37.3, five with spills 35.7; no early trigger 34.8; with five CTAs also no early
+// trigger 37.8, no programmatic launches 39.0.
 struct TFirst {
     int flux;                  // records with fluxes of the largest tile, rounded up to 4
     int grad;                  // core and ring-1 cells of the largest tile
@@ -1011,8 +1011,8 @@ __global__ void __launch_bounds__(kTileCore, 4) k_tfirst(TArgs a, TFirst f) {
 // Such a solve is bound by latency, not by any unit: with a stage kernel per stage it spends ~15 us a
 // stage on the launch, the tile's block copies and a 256-cell tile's passes on a third of the SMs.
 // Here a stage is the barrier and the ring gather (~1.5 us), one round of gradients and fluxes and
-// the update: 12k-cell NS cylinder 45.1 -> 16.5 us per iteration, 50k Euler polygons 42.5 -> 19.2, 512
-// quads 26.6 -> 11.8.  What the passes read every stage (LSQ moments, previous states) is kept in shared
+// the update: 12k-cell NS cylinder 45.1 -> 16.1 us per iteration, 50k Euler polygons 42.5 -> 19.2, 512
+// quads 26.6 -> 11.7.  What the passes read every stage (LSQ moments, previous states) is kept in shared
 // memory too, since the barrier's acquire empties L1 (the 12k-cell cylinder: 19.8 -> 16.7
 // us when it was added, with a barrier that has no fences beyond its release and acquire).  MINB 2 has the
 // registers to run without spills; MINB 3 (128 B of spills) takes the solves whose tiles do not fit two to

@@ -31,7 +31,9 @@ extern "C" {
 #define FV2D_ERR_STATE      7   /* non-physical state detected (NaN, rho <= 0 or P <= 0)        */
 #define FV2D_ERR_NODEV      8   /* no CUDA device / the library's kernels cannot run here       */
 
-#define FV2D_FP64 0             /* plain FP64 path, bit-exact with the reference                */
+/* plain FP64 path, bit-exact with the reference; on Arm hosts the freestream energy that the case's
+ * rho, u, v, P give may be an ulp off the reference's (about 5 % of inputs; host compiler's contraction) */
+#define FV2D_FP64 0
 #define FV2D_FP32 1             /* FP32 state/gradients/fluxes; LSQ terms from FP64; FP64 norms */
 
 /* Codes as read_inputs maps them (src/base/read_inputs.cpp:44-206). */
@@ -174,6 +176,8 @@ int fv2d_set_store_residual(fv2d_handle* h, int every_stage);
 int fv2d_set_graphs(fv2d_handle* h, int enable);
 /* Time every kernel launch with CUDA events on the handle's stream (off by default).          */
 int fv2d_set_kernel_timing(fv2d_handle* h, int enable);
+/* Timed FP32 steps run one kernel per RK stage also where untimed ones take whole iterations in one
+ * launch (solves whose tiles all fit on the GPU: about 2.5 times less per iteration).          */
 /* Per-kernel totals since timing was enabled: names (comma separated into buf), ms, launches. */
 int fv2d_kernel_times(fv2d_handle* h, char* names, int names_len, double* ms, int* launches, int max_kernels, int* n_kernels);
 /* The handle's CUDA stream (a cudaStream_t), for callers that order their own work after it.  */
