@@ -113,15 +113,16 @@ inline bool host_pinned(const void* p) {
 // host (pageable) -> device through `stage` (pinned, >= bytes); returns the first CUDA error.
 // `stage_free` is recorded after the last DMA and waited on before the staging buffer is written
 // again, so a second upload never overwrites data an earlier one has not transferred yet.
-// A page-locked `host` is read by the DMA itself: `*reading` (when given) says so, and the caller's
-// buffer must not be handed back before `stage_free` has passed.
+// A page-locked `host` is read by the DMA itself, and the caller's buffer must not be handed back before
+// that is over: `*reading` (when given) says so and `stage_free` is recorded behind it; a caller that waits
+// for the stream anyway gives none.
 inline cudaError_t staged_h2d(void* dev, const void* host, size_t bytes, void* stage, cudaStream_t s,
                               cudaEvent_t stage_free, bool* reading = nullptr) {
     const bool direct = host_pinned(host);
     if (reading) *reading = direct;
     if (direct) {
         const cudaError_t e = cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, s);
-        return e == cudaSuccess ? cudaEventRecord(stage_free, s) : e;
+        return e == cudaSuccess && reading ? cudaEventRecord(stage_free, s) : e;
     }
     cudaError_t e = cudaEventSynchronize(stage_free);
     for (size_t off = 0; e == cudaSuccess && off < bytes; off += kCopyChunk) {

@@ -181,8 +181,10 @@ public:
         const size_t ohalo = take(4 * (size_t)c.halo);
         const size_t otiles = take(sizeof(TileDesc) * (size_t)c.tiles), otpart = take(32 * (size_t)c.tiles);
         const size_t oP = take(sizeof(TParams) * (size_t)c.solves), osmax = take(4 * (size_t)c.solves);
-        const size_t oflag = take(4 * (size_t)c.solves), ores = take(32 * (size_t)c.solves);
-        const size_t osr = take(8 * (size_t)c.solves), omisc = take(256);
+        const size_t ores = take(32 * (size_t)c.solves), osr = take(8 * (size_t)c.solves);
+        // (the error word, in misc, follows the flags; the barrier word, in misc too, stays apart from smax, which a
+        // stage's last warps add to: 512 bytes nearer, 50k polygons took 1 % more)
+        const size_t oflag = take(4 * (size_t)c.solves), omisc = take(256);
         bytes_ = off;
         FV2D_T(cudaMalloc(&arena_, bytes_));
         char* a = (char*)arena_;
@@ -968,8 +970,9 @@ public:
         FV2D_T(cudaMemcpyAsync(n2o, s.image->pin + s.image->o_n2o, 4 * (size_t)s.n, cudaMemcpyHostToDevice, st));
         k_state_out<float><<<(unsigned)((s.n + 255) / 256), 256, 0, st>>>((int)s.n, 4, n2o, A.Q[0] + s.c0, out, A.Qlo + s.c0);
         FV2D_T(cudaGetLastError());
-        FV2D_T(cudaMemcpyAsync(flag_pin_, A.flags + sid, 4, cudaMemcpyDeviceToHost, st));
-        FV2D_T(cudaMemcpyAsync(flag_pin_ + 1, A.err, 4, cudaMemcpyDeviceToHost, st));
+        // the flag and the error word, which follows the flags in the arena, as two rows of one copy
+        FV2D_T(cudaMemcpy2DAsync(flag_pin_, 4, A.flags + sid, (size_t)((const char*)A.err - (const char*)(A.flags + sid)), 4, 2,
+                                 cudaMemcpyDeviceToHost, st));
         const size_t bytes = 32 * (size_t)s.n;
         if (host_pinned(q)) {
             FV2D_T(cudaMemcpyAsync(q, out, bytes, cudaMemcpyDeviceToHost, st));
