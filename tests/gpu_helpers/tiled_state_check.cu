@@ -1,5 +1,5 @@
-// Test harness: the FP32 engine's batch with its members open, for what no entry point can bring about
-// without a fault: the kernels' error word set from the host.
+// Test harness: the FP32 engine with its members open: the kernels' error word set from the host (what no
+// entry point can bring about without a fault), and which kernels a step takes.
 #include <algorithm>
 #include <condition_variable>
 #include <cstdio>
@@ -31,5 +31,24 @@ int batch_with_error(const fv2d_mesh_desc* d, const fv2d_case* cs, int bits, int
     *norms = b->norms(&id, nr, &it, 1, &n);
     *sync = b->synchronize();
     return 0;
+}
+
+static int path_of(const fv2d::TiledCore& c) {
+    return c.iter_fn_ == (const void*)fv2d::k_titer<2> ? 2 : c.iter_fn_ == (const void*)fv2d::k_titer<3> ? 3 : c.first_ ? 1 : 0;
+}
+// What steps run, after one: 0 the general stage kernels, 1 the first-order ones, 2 and 3 whole iterations
+// with two and three tiles per SM; -1 on an error.  For a single solve, and for a batch of a solve of each case.
+int solver_path(const fv2d_mesh_desc* d, const fv2d_case* cs) {
+    fv2d::TiledSolver s;
+    std::string err;
+    if (fv2d::build_mesh(d, cs, s.mesh_, err, s.side_block(d->num_cells)) || s.init(*cs) || s.step(1) || s.synchronize()) return -1;
+    return path_of(s.core_);
+}
+int batch_path(const fv2d_mesh_desc* d, const fv2d_case* cases, int n) {
+    fv2d::TiledBatch b;
+    if (b.init((long long)n * (d->num_cells + 64), (long long)n * (d->num_faces + 64), n)) return -1;
+    for (int i = 0, sid; i < n; i++)
+        if (b.add(d, cases + i, &sid)) return -1;
+    return b.step(1) || b.synchronize() ? -1 : path_of(b.core_);
 }
 }

@@ -1,4 +1,5 @@
-"""FP32 batches: a kernel that gave up (a copy or a barrier that timed out, a refused descriptor) leaves its
+"""The FP32 engine's inside: which kernels a step takes (so that tests which compare them compare what they say),
+and in batches: a kernel that gave up (a copy or a barrier that timed out, a refused descriptor) leaves its
 tiles at different stages; every call that returns results reports it."""
 import ctypes
 import glob
@@ -41,3 +42,21 @@ def test_kernel_errors_reach_the_caller(pkg, helper, bits, words, order):
     assert helper.batch_with_error(ctypes.byref(d.desc), ctypes.byref(cs), bits, *[ctypes.byref(r) for r in rc], msg, 256) == 0
     assert [bool(r.value) for r in rc] == [bits != 0] * 3
     assert len({r.value for r in rc}) == 1 and words in msg.value.decode()
+
+
+@pytest.mark.parametrize("kind,size,order,path", [
+    ("quads", (5, 4), 1, 2), ("quads", (139, 70), 1, 2), ("bump", 9000, 1, 2), ("bump", 76000, 1, 2), ("bump", 84000, 1, 3),
+    ("bump", 130000, 1, 0), ("quads", (5, 4), 0, 1), ("bump", 9000, 0, 1)])
+def test_kernels_of_a_solve(pkg, helper, kind, size, order, path):
+    mg = pkg.meshgen
+    grid = mg.channel_bump_quads(*size) if kind == "quads" else mg.voronoi_bump_channel(size, seed=3)
+    d = pkg.fv2d._Desc(grid)
+    _, cs = mesh_case(pkg, solution_poly_order=order)
+    assert helper.solver_path(ctypes.byref(d.desc), ctypes.byref(cs)) == path
+
+
+@pytest.mark.parametrize("orders,path", [((1,), 2), ((1, 0), 2), ((0, 0), 1), ((0, 1, 1), 2)])
+def test_kernels_of_a_batch(pkg, helper, orders, path):
+    d, _ = mesh_case(pkg)
+    cases = (pkg.Case * len(orders))(*[mesh_case(pkg, solution_poly_order=o)[1] for o in orders])
+    assert helper.batch_path(ctypes.byref(d.desc), cases, len(orders)) == path
